@@ -38,23 +38,35 @@ def nvcc() -> str:
     raise RuntimeError("nvcc not found")
 
 
-def sources() -> list[Path]:
-    return sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cpp")))
+# the fast sweep's kernels: one translation unit per coefficient form and
+# tile height (each takes tens of seconds; in one file they would be serial)
+FAST = CSRC / "tti_fast_inst.cu"
+FAST_UNITS = [(form, ty) for form in ("CF_F32", "CF_F16", "CF_BF16", "CF_VV") for ty in (8, 16)]
+
+
+def sources() -> list[tuple[Path, list[str], str]]:
+    """(source, defines, object name) of every translation unit, the slow
+    ones first."""
+    units = [(FAST, [f"-DDC_FORM={form}", f"-DDC_TY={ty}"], f"{FAST.stem}_{form}_{ty}.o")
+             for form, ty in FAST_UNITS]
+    rest = sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cpp")))
+    return units + [(s, [], s.name + ".o") for s in rest if s != FAST]
 
 
 def _headers() -> list[Path]:
     return list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
 
 
-def _compile(src: Path) -> Path:
-    obj = BUILD / (src.name + ".o")
+def _compile(unit: tuple[Path, list[str], str]) -> Path:
+    src, defines, name = unit
+    obj = BUILD / name
     deps = [src] + _headers()
     if obj.exists() and all(d.stat().st_mtime <= obj.stat().st_mtime for d in deps):
         return obj
     flags = COMMON + ARCH
     if src.suffix == ".cpp":
         flags = COMMON + HOST_STRICT
-    cmd = [nvcc(), "-c", str(src), "-o", str(obj), *flags]
+    cmd = [nvcc(), "-c", str(src), "-o", str(obj), *flags, *defines]
     if os.environ.get("DC_GB300_PTXAS_VERBOSE"):
         cmd += ["-Xptxas", "-v"]
     proc = subprocess.run(cmd, capture_output=True, text=True)
@@ -78,7 +90,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if force:
         for o in BUILD.glob("*.o"):
             o.unlink()
-    with cf.ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with cf.ThreadPoolExecutor(max_workers=min(os.cpu_count() or 8, len(srcs))) as ex:
         objs = list(ex.map(_compile, srcs))
     if LIB.exists() and all(o.stat().st_mtime <= LIB.stat().st_mtime for o in objs):
         build_cli()

@@ -172,7 +172,6 @@ struct Sim {
   int config_version = 0;
   // tensor maps for the fast kernel (encoded for one tile shape)
   CUtensorMap tm_halo[2], tm_own[2], tm_c[4];  // tm_c: L, O1, O2, row bases
-  bool deep_ring = false;  // fast FP32 sweep with the 4-stage TMA ring
   int fast_slots = 0;      // fast-sweep CTAs resident on the device at once
   int maps_tx = 0, maps_ty = 0;
   // learned absorbing layer, applied after every stencil pass of a run
@@ -191,6 +190,32 @@ struct Sim {
   int graph_version[2] = {-1, -1};
   int graph_pc[2] = {-1, -1};
 };
+
+// The kernels of the fast sweep for one coefficient form and tile height:
+// tti_fast_inst.cu is compiled once per pair and specialises fast_ops.
+struct FastOps {
+  cudaError_t (*attrs)();  // shared-memory attributes
+  int (*occupancy)();      // CTAs per SM
+  cudaError_t (*launch)(Sim *sim, const StepParams &prm, int cur_buf, int prev_buf);
+  cudaError_t (*batch_attrs)();
+  int (*batch_occupancy)(bool iso, bool sponge);
+  cudaError_t (*launch_batch)(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
+                              int blocks);
+};
+constexpr int kFastTX = 32;  // tile width: half a warp of two-point lanes
+constexpr int kGroup = 3;    // planes of a TMA copy, and between two CTA barriers
+template <int FORM, int TY>
+const FastOps &fast_ops();
+#define DCG_DECL_OPS(f)              \
+  template <>                        \
+  const FastOps &fast_ops<f, 8>();   \
+  template <>                        \
+  const FastOps &fast_ops<f, 16>()
+DCG_DECL_OPS(CF_F32);
+DCG_DECL_OPS(CF_VV);
+DCG_DECL_OPS(CF_F16);
+DCG_DECL_OPS(CF_BF16);
+#undef DCG_DECL_OPS
 
 // Fast-kernel tile geometry (chosen at compile time; see tti_fast.cu).
 struct FastShape {
