@@ -22,10 +22,9 @@ const FastOps &ops_for(int form, int ty) {
   }
 }
 
-// 32 x 8 tiles with two CTAs per SM measured fastest on GB300 (616^3 cube:
-// 2.83 ms per step vs 3.09 ms for 32 x 16; 32 x 6 with three CTAs per SM
-// was slower still: 2.93 ms FP32, 2.68 ms FP16 against 2.56 ms).
-// DC_GB300_FAST_TY=16 selects 32 x 16.
+// 32 x 8 tiles (two CTAs of 128 threads per SM): with 32 x 16 and one CTA of
+// 256 threads per SM nothing runs while a CTA waits at its barrier or fills
+// its queues.  DC_GB300_FAST_TY=16 selects 32 x 16.
 int chosen_ty(int) {
   const char *e = std::getenv("DC_GB300_FAST_TY");
   const int v = e ? std::atoi(e) : 0;

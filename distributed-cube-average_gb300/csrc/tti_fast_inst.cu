@@ -6,14 +6,15 @@
 // reference, include/sample_compute.h:105-185) for every point of a box.
 //
 // Work decomposition: a CTA owns a 32 x TY column tile in (x, y) and sweeps
-// a chunk of output planes along z.  For the leading plane k it receives,
-// by TMA into a 3-deep shared-memory ring:
-//   * the (p, q) pairs of plane k with a 4-cell halo in x and y and the
-//     in-plane coefficient group (cxx, cyy, cxy, czz) of plane k,
-//   * the other coefficients and the (pp, qp) tile of the output plane
+// a chunk of output planes along z.  It receives by TMA, a group of three
+// planes per copy into one of two shared-memory stages:
+//   * the (p, q) pairs of the leading planes k with a 4-cell halo in x and y
+//     and the in-plane coefficient group (cxx, cyy, cxy, czz) of plane k,
+//   * the other coefficients and the (pp, qp) tile of the output planes
 //     z = k - 4.
-// Each thread owns one (x, y) column and keeps, in registers, 9-deep queues
-// of (p, q) pairs: the centre value, the x-derivative and the y-derivative.
+// Each lane owns two x-adjacent columns and keeps, in registers, the (p, q)
+// pairs of the last eight planes: the centre value, the x-derivative and the
+// y-derivative.
 // The cross derivatives are evaluated in their separable form: with the
 // 8th-order first-derivative weights L1..L4 the reference's 64-point
 // derCross (include/derivatives.h:56-91) has weights L_ab = L_a * L_b, so it
@@ -22,13 +23,34 @@
 //   d2/dxdz = D_z of the x-derivative queue,
 //   d2/dydz = D_z of the y-derivative queue.
 // The in-plane part of H1 (cxx d2/dx2 + cyy d2/dy2 + cxy d2/dxdy), the
-// in-plane Laplacian and czz of plane k wait four planes in a per-thread
-// shared-memory ring (9 slots, indexed by the compile-time plane number)
-// until plane k is the output plane.
+// in-plane Laplacian and czz of plane k wait four planes in registers until
+// plane k is the output plane.
+//
+// What bounds it, and why this shape.  Next to HBM the shared-memory pipe and
+// the instruction issue of the few resident warps count: with one column per
+// lane (16 warps per SM, 114 registers, one barrier per plane) a 304^3 FP16
+// step took 347 us at 70 % of the shared-memory wavefronts and 268
+// instructions per 32 points, 107 of them addresses, branches and barriers.
+//   * Two adjacent columns share their row's values: five 16-byte loads bring
+//     ten pairs instead of eighteen 8-byte ones, and four the y-derivatives
+//     around both: 89 -> 59 wavefronts per 32 points.  The queues of two
+//     columns (up to 255 registers) leave 8 warps per SM.
+//   * A warp owns two whole tile rows, so the y-derivative plane is exchanged
+//     inside a warp and the CTA meets at a barrier once per group.  One copy
+//     per array and group: a third of the TMA instructions, one wait.
+//   * The unrolled body is one group (three planes) and the queues move by
+//     three planes at its end.  Unrolled over the nine planes of a register
+//     ring nothing moves, but the 50 KB body misses the instruction cache:
+//     0.84 of 4.4 stall cycles per instruction, 286 against 264 us (six
+//     planes: 282 us).
+// 304^3 FP16 step 347 -> 264 us (ncu), 616^3 FP32 step 2.59 -> 2.19 ms (96 %
+// of the measured copy bandwidth), 872 x 872 x 616 FP16 5.19 -> 3.79 ms;
+// loading the next plane's values ahead of the output arithmetic ran out of
+// registers (282 us).
 //
 // The sweep of one column tile is `sweep_column`; `fast_kernel` runs one
-// tile per CTA over one box, `batch_kernel` runs persistent CTAs over the
-// tiles of many boxes (shots) cropped out of one shared medium.
+// tile per CTA over one box, `batch_kernel` runs CTAs over the tiles of many
+// boxes (shots) cropped out of one shared medium.
 // Rounding differs from the reference's direct sums (the exact kernel is
 // bit-identical).
 //
@@ -149,9 +171,10 @@ constexpr float kL1 = 4.0f / 5.0f, kL2 = -1.0f / 5.0f, kL3 = 4.0f / 105.0f,
 
 // Two forms of each derivative with the constant weights: two FMA chains
 // summed at the end (shorter dependency chains), or one chain (one
-// instruction fewer).  The FP16/BF16 sweeps run 2 % faster with the second
-// (64-shot FP16 batch: 32.57 vs 33.19 ms); the FP32-medium sweep, nearer its
-// memory bound, gains nothing from it and keeps the first.
+// instruction fewer).  The FP16/BF16 sweeps use the second (with one column
+// per lane it was 2 % faster: 64-shot FP16 batch 32.57 vs 33.19 ms); the
+// FP32-medium sweep, nearer its memory bound, gained nothing and keeps the
+// first.
 template <bool CHAIN>
 __device__ __forceinline__ float2 d2k(float2 c, float2 m1, float2 p1, float2 m2, float2 p2,
                                       float2 m3, float2 p3, float2 m4, float2 p4) {
@@ -220,15 +243,22 @@ __device__ __forceinline__ float2 h2f(uint32_t v, bool bf16) {
 }
 
 // Two 16-bit fixed-point values (low half first, each stored biased by
-// 2^15 and scaled by 2^15) as exact floats: a byte permutation places each
-// half in the low mantissa bits of 2^23, and one packed multiply-add removes
-// scale and offset (2^23 + 2^15) / 2^15 = 257; every step is exact.
+// 2^15) as exact floats: a byte permutation places each half in the low
+// mantissa bits of 2^23, and one packed subtraction of 2^23 + 2^15 removes
+// both offsets.  The values come out scaled by 2^15; the sweep unscales H1
+// once (unscaling here instead costs the same and rounds differently where
+// the products are subnormal, at the far fringe of a wave).
 __device__ __forceinline__ float2 fx2f(uint32_t w) {
   const uint32_t lo = __byte_perm(w, 0x4b000000u, 0x7610);
   const uint32_t hi = __byte_perm(w, 0x4b000000u, 0x7632);
-  return __ffma2_rn(make_float2(__uint_as_float(lo), __uint_as_float(hi)),
-                    make_float2(1.0f / 32768.0f, 1.0f / 32768.0f), make_float2(-257.0f, -257.0f));
+  return __fadd2_rn(make_float2(__uint_as_float(lo), __uint_as_float(hi)),
+                    make_float2(-8421376.0f, -8421376.0f));
 }
+
+// Scale of the angle terms as the kernel reads them (1 / 2^15 for the
+// fixed-point FP16 form, applied to H1).
+template <int CF>
+constexpr float kChUnscale = CF == CF_F16 ? 1.0f / 32768.0f : 1.0f;
 
 // Shared-memory loads and stores at a 32-bit address plus a compile-time
 // offset, so every access of the unrolled sweep is one instruction on a
@@ -361,8 +391,8 @@ __device__ __forceinline__ void load_out(const StageAddr &sa, OutMedium out[2]) 
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       if (CF == CF_F16) {
-        // fixed-point cxz, cyz; velocity v = b + b * d from the row's bases
-        // vb and the FP16 ratios d
+        // fixed-point cxz, cyz (x 2^15); velocity v = b + b * d from the row's
+        // bases vb and the FP16 ratios d
         const float2 a = fx2f(w1[2 * k]), b = h2f(w1[2 * k + 1], false), c = h2f(w2[k], false);
         out[k] = OutMedium{a.x, a.y, fmaf(vb.x, b.x, vb.x), fmaf(vb.y, b.y, vb.y),
                            fmaf(vb.z, c.x, vb.z), fmaf(vb.w, c.y, vb.w)};
@@ -396,7 +426,6 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
   constexpr int HX = Lay::HX;
   constexpr int NT = Lay::NT;
   constexpr unsigned kAll = 0xffffffffu;
-  static_assert(9 % GROUP == 0, "the 9-plane body holds whole groups");
   // single-chain derivatives for the narrow-coefficient sweeps (see d2k)
   constexpr bool CHAIN = CF == CF_F16 || CF == CF_BF16;
   // equal spacing on all axes: one set of weights serves x, y and z
@@ -458,12 +487,13 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
 
   if (tid == 0) issue(0, 0);
 
-  // Register queues of (p, q) pairs indexed by plane mod 9 (compile-time
-  // after unrolling): centre value, x- and y-derivative of both points, and
-  // the delayed in-plane terms (A: in-plane part of H1, B: in-plane
-  // Laplacian, czz) of the last four planes.
-  float2 cq[9][2], dxq[9][2], dyq[9][2], aq[9][2], bq[9][2];
-  float zq[9][2];
+  // Register queues of both columns.  cq, dxq, dyq: centre value, x- and
+  // y-derivative of the last eight planes (oldest first) and of the body's
+  // own; aq, bq, zq: in-plane part of H1, in-plane Laplacian and czz of the
+  // last four and the body's own.  Moved down by GROUP after every body.
+  float2 cq[8 + GROUP][2], dxq[8 + GROUP][2], dyq[8 + GROUP][2];
+  float2 aq[kHalo + GROUP][2], bq[kHalo + GROUP][2];
+  float zq[kHalo + GROUP][2];
   float2 e_acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
   bool bad = false;  // a wait of this thread timed out
 
@@ -498,16 +528,17 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
   const uint32_t sbase = smem_u32(smem);
   StageAddr sa;
   sa.halo = sbase + Lay::OFF_H + 8 * ((ty + kHalo) * HX + tx + kHalo);
-  // the halo column whose y-derivative this lane computes (lanes 0-15: four
-  // columns on either side of the warp's two rows)
+  // the halo column whose y-derivative this lane computes (four columns on
+  // either side of the warp's two rows; lanes 16-31: of the next plane)
   const int hrow = 2 * warp + ((lane >> 3) & 1), hcol = (lane & 7) < 4 ? (lane & 7) : TX + (lane & 7);
-  sa.col = sbase + Lay::OFF_H + 8 * ((hrow + kHalo) * HX + hcol);
+  sa.col = sbase + Lay::OFF_H + 8 * ((hrow + kHalo) * HX + hcol) + (lane < 16 ? 0 : Lay::H_PLANE);
   sa.t8 = sbase + 8 * (ty * TX + tx);
   sa.t4 = sbase + 4 * (ty * TX + tx);
   sa.t16 = (sbase + 16 * (ty * TX + tx)) ^ ((tid & 4) ? 16u : 0u);
   sa.row = sbase + 16 * ty;
   const uint32_t dy = sbase + Lay::OFF_DY + 8 * (ty * HX + tx + kHalo);
-  const uint32_t dycol = sbase + Lay::OFF_DY + 8 * (hrow * HX + hcol);
+  const uint32_t dycol =
+      sbase + Lay::OFF_DY + 8 * (hrow * HX + hcol) + (lane < 16 ? 0 : Lay::DY_BYTES);
   // global position of the first point at the first output plane (advanced
   // by one plane per output; never dereferenced for inactive points)
   float2 *out = prm.prev + (static_cast<long long>(zb) * prm.plane +
@@ -516,23 +547,22 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
   int sel = 1;        // stage of the current group
   uint32_t par = 1u;  // its mbarrier parity
   sa.shift(Lay::STAGE_BYTES);
-  int it0 = 0;      // first iteration of the 9-plane body
+  int it0 = 0;      // first iteration of the body (one group)
   int stop = n_it;  // a group boundary where a time-out was seen
 
-  // Iteration it0 + u; false at the end of the sweep.
+  // Iteration it0 + u; false past the end of the sweep.
   auto plane = [&](auto U) __attribute__((always_inline)) {
     constexpr int u = decltype(U)::value;
-    constexpr int g = u % GROUP;  // the plane inside its group
-    constexpr int DY = (u % 3) * Lay::DY_BYTES;
+    constexpr int DY = u * Lay::DY_BYTES;
     if (it0 + u >= n_it) return false;  // CTA-uniform
-    if (g == 0) {
+    if (u == 0) {
       // Every warp has read the previous group: refill its stage with the
       // next one, then wait for the current one.
       if (__syncthreads_or(bad)) {
-        stop = it0 + u;
+        stop = it0;
         return false;
       }
-      if (tid == 0 && it0 + u + GROUP < n_it) issue(it0 + u + GROUP, sel);
+      if (tid == 0 && it0 + GROUP < n_it) issue(it0 + GROUP, sel);
       sa.shift(sel ? -Lay::STAGE_BYTES : Lay::STAGE_BYTES);
       sel ^= 1;
       par ^= sel ^ 1;
@@ -548,7 +578,7 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
     float2 xx[2], yy[2];
     {
       float2 w[10], v[8][2];  // row of the two points; their columns
-      constexpr int H = Lay::OFF_H + g * Lay::H_PLANE;
+      constexpr int H = Lay::OFF_H + u * Lay::H_PLANE;
       ld_pairs<H - 32>(sa.halo, w[0], w[1]);
       ld_pairs<H - 16>(sa.halo, w[2], w[3]);
       ld_pairs<H>(sa.halo, w[4], w[5]);
@@ -565,36 +595,36 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const float2 m = w[4 + c];
-        cq[u][c] = m;
-        dyq[u][c] = d1s<ISO, CHAIN>(w1y, v[3][c], v[4][c], v[2][c], v[5][c], v[1][c], v[6][c],
+        cq[8 + u][c] = m;
+        dyq[8 + u][c] = d1s<ISO, CHAIN>(w1y, v[3][c], v[4][c], v[2][c], v[5][c], v[1][c], v[6][c],
                                     v[0][c], v[7][c]);
         yy[c] = d2s<ISO, CHAIN>(w2y, m, v[3][c], v[4][c], v[2][c], v[5][c], v[1][c], v[6][c],
                                 v[0][c], v[7][c]);
         xx[c] = d2s<ISO, CHAIN>(w2x, m, w[3 + c], w[5 + c], w[2 + c], w[6 + c], w[1 + c],
                                 w[7 + c], w[c], w[8 + c]);
-        dxq[u][c] = d1s<ISO, CHAIN>(w1x, w[3 + c], w[5 + c], w[2 + c], w[6 + c], w[1 + c],
+        dxq[8 + u][c] = d1s<ISO, CHAIN>(w1x, w[3 + c], w[5 + c], w[2 + c], w[6 + c], w[1 + c],
                                     w[7 + c], w[c], w[8 + c]);
       }
-      sts4<DY>(dy, dyq[u][0], dyq[u][1]);
-      // y-derivatives of the 4 + 4 halo columns (needed by d2/dxdy)
-      if (lane < 16)
+      sts4<DY>(dy, dyq[8 + u][0], dyq[8 + u][1]);
+      // y-derivatives of the 4 + 4 halo columns (needed by d2/dxdy): of this
+      // plane and the next one at once where the group holds both
+      if (u % 2 == 0 && (u + 1 < GROUP || lane < 16))
         sts2<DY>(dycol, d1s<ISO, CHAIN>(w1y, lds2<H - 8 * HX>(sa.col), lds2<H + 8 * HX>(sa.col),
                                         lds2<H - 16 * HX>(sa.col), lds2<H + 16 * HX>(sa.col),
                                         lds2<H - 24 * HX>(sa.col), lds2<H + 24 * HX>(sa.col),
                                         lds2<H - 32 * HX>(sa.col), lds2<H + 32 * HX>(sa.col)));
     }
 
-    // ---- output plane z = k - 4, from the ninth iteration on
-    if (u == 8 || it0 > 0) {
+    // ---- output plane z = k - 4
+    if (it0 + u >= 2 * kHalo) {
       // queue slots of planes z-4 .. z+4
-      constexpr int m4 = (u + 1) % 9, m3 = (u + 2) % 9, m2 = (u + 3) % 9, m1 = (u + 4) % 9,
-                    z0 = (u + 5) % 9, p1 = (u + 6) % 9, p2 = (u + 7) % 9, p3 = (u + 8) % 9,
-                    p4 = u;
+      constexpr int m4 = u, m3 = u + 1, m2 = u + 2, m1 = u + 3, z0 = u + 4, p1 = u + 5,
+                    p2 = u + 6, p3 = u + 7, p4 = u + 8;
       OutMedium md[2];
-      load_out<CF, Lay::OFF_O1 + g * Lay::O1_PLANE, Lay::OFF_O2 + g * Lay::O2_PLANE,
-               Lay::OFF_VB + g * Lay::VB_PLANE>(sa, md);
+      load_out<CF, Lay::OFF_O1 + u * Lay::O1_PLANE, Lay::OFF_O2 + u * Lay::O2_PLANE,
+               Lay::OFF_VB + u * Lay::VB_PLANE>(sa, md);
       float2 pv[2], nv[2];
-      ld_pairs<Lay::OFF_OWN + g * Lay::OWN_PLANE>(sa.t8, pv[0], pv[1]);
+      ld_pairs<Lay::OFF_OWN + u * Lay::OWN_PLANE>(sa.t8, pv[0], pv[1]);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const float2 zz = d2s<ISO, CHAIN>(w2z, cq[z0][c], cq[m1][c], cq[p1][c], cq[m2][c],
@@ -605,9 +635,10 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
                                           dyq[m3][c], dyq[p3][c], dyq[m4][c], dyq[p4][c]);
         // H1 = sum c * d2 over the six second derivatives; the Laplacian
         // (H1 + H2) = xx + yy + zz
-        const float2 h1 = fma2(bc(md[c].cyz), yz,
-                               fma2(bc(md[c].cxz), xz, fma2(bc(zq[z0][c]), zz, aq[z0][c])));
-        const float2 h2 = fma2(bc(-1.0f), h1, add2(bq[z0][c], zz));
+        float2 h1 = fma2(bc(md[c].cyz), yz,
+                         fma2(bc(md[c].cxz), xz, fma2(bc(zq[u][c]), zz, aq[u][c])));
+        if (CF == CF_F16) h1 = mul2(h1, bc(kChUnscale<CF>));
+        const float2 h2 = fma2(bc(-1.0f), h1, add2(bq[u][c], zz));
         const float rhsp =
             fmaf(md[c].v2sz, h1.x - h1.y, fmaf(md[c].v2pz, h1.y, md[c].v2px * h2.x));
         const float rhsq =
@@ -665,7 +696,7 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
     }
 
     // ---- in-plane part of H1 (A) and of the Laplacian (B) at plane k; they
-    // wait in queue slot u for 4 planes.  The dy rows are the warp's own:
+    // wait in the queues for 4 planes.  The dy rows are the warp's own:
     // only its lanes have to have stored them.  (Before iteration 4 and in
     // the last four the slot is never read: whatever the stage holds will
     // do.)
@@ -676,27 +707,40 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
       ld_pairs<DY - 16>(dy, e[2], e[3]);
       ld_pairs<DY + 16>(dy, e[6], e[7]);
       ld_pairs<DY + 32>(dy, e[8], e[9]);
-      e[4] = dyq[u][0];
-      e[5] = dyq[u][1];
+      e[4] = dyq[8 + u][0];
+      e[5] = dyq[8 + u][1];
       float4 lc[2];
-      load_lead<CF, Lay::OFF_L + g * Lay::L_PLANE>(sa, lc);  // cxx, cyy, cxy, czz
+      load_lead<CF, Lay::OFF_L + u * Lay::L_PLANE>(sa, lc);  // cxx, cyy, cxy, czz
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const float2 xy = d1s<ISO, CHAIN>(w1x, e[3 + c], e[5 + c], e[2 + c], e[6 + c], e[1 + c],
                                           e[7 + c], e[c], e[8 + c]);
-        aq[u][c] = fma2(bc(lc[c].z), xy, fma2(bc(lc[c].y), yy[c], mul2(bc(lc[c].x), xx[c])));
-        bq[u][c] = add2(xx[c], yy[c]);
-        zq[u][c] = lc[c].w;
+        aq[kHalo + u][c] = fma2(bc(lc[c].z), xy, fma2(bc(lc[c].y), yy[c], mul2(bc(lc[c].x), xx[c])));
+        bq[kHalo + u][c] = add2(xx[c], yy[c]);
+        zq[kHalo + u][c] = lc[c].w;
       }
     }
     return true;
   };
-  while (plane(Const<0>{}) && plane(Const<1>{}) && plane(Const<2>{}) && plane(Const<3>{}) &&
-         plane(Const<4>{}) && plane(Const<5>{}) && plane(Const<6>{}) && plane(Const<7>{}) &&
-         plane(Const<8>{})) {
-    it0 += 9;
-    ev -= 9;
-    if (SPONGE) gzp += 9;
+  while (plane(Const<0>{}) && plane(Const<1>{}) && plane(Const<2>{})) {
+    it0 += GROUP;
+    ev -= GROUP;
+    if (SPONGE) gzp += GROUP;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        cq[i][c] = cq[i + GROUP][c];
+        dxq[i][c] = dxq[i + GROUP][c];
+        dyq[i][c] = dyq[i + GROUP][c];
+      }
+#pragma unroll
+      for (int i = 0; i < kHalo; ++i) {
+        aq[i][c] = aq[i + GROUP][c];
+        bq[i][c] = bq[i + GROUP][c];
+        zq[i][c] = zq[i + GROUP][c];
+      }
+    }
   }
   if (__syncthreads_or(bad)) {
     // A TMA wait timed out: record it, give the copies still in flight a

@@ -1,0 +1,74 @@
+"""The fast sweep at the edges of its decomposition: tiles of 32 x 8 with two
+columns per lane, groups of three planes, chunks of any length.
+
+Fields: rel. L2 to the exact kernel on the same inputs <= 1e-5 (both compute
+the same sums in FP32; a few steps apart by some units of 2^-24 each).
+Traces: the values the kernel stored, so equal to the fields bit for bit.
+"""
+import numpy as np
+import pytest
+
+from oracle.oracle import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# (9: one updated point; odd and even ends of a lane's pair; one column or row
+# past a full tile; 1, 2 and 0 planes past a full group)
+SIZES = [(9, 9, 9), (10, 11, 10), (13, 9, 14), (41, 17, 11), (42, 16, 12), (73, 25, 13),
+         (40, 24, 46)]
+
+
+def inputs(sizes, seed):
+    rng = np.random.default_rng(seed)
+    shape = sizes[::-1]
+    coef = [rng.uniform(-0.5, 0.5, shape).astype(np.float32) for _ in range(6)]
+    coef += [rng.uniform(4e6, 9e6, shape).astype(np.float32) for _ in range(4)]
+    fields = []
+    for _ in range(4):
+        f = np.zeros(shape, np.float32)
+        f[4:-4, 4:-4, 4:-4] = rng.standard_normal([s - 8 for s in shape])
+        fields.append(f)
+    return coef, fields
+
+
+def run(dc, sizes, kernel, medium, coef, fields, src, rec, steps, sponge, d):
+    with dc.Simulation(sizes, d, 1e-3, kernel=kernel, medium=medium, device=0) as sim:
+        if medium == dc.MEDIUM_PRECOMP:
+            sim.set_precomp(coef)
+        else:
+            sim.set_vpz_vsv(np.sqrt(coef[6]), 0.4 * np.sqrt(coef[7]))
+        sim.set_fields(*fields)
+        sim.set_source(src, np.linspace(1.0, 2.0, steps + 1))
+        if sponge:
+            sim.set_sponge(*(np.linspace(0.9, 1.0, n) for n in sizes))
+        sim.set_receivers(rec, steps)
+        sim.enable_energy(steps)
+        sim.run(steps)
+        sim.synchronize()
+        return sim.get_fields(), sim.traces(steps), sim.energy(steps)
+
+
+@pytest.mark.parametrize("sponge", [False, True])
+@pytest.mark.parametrize("even", [True, False])
+@pytest.mark.parametrize("sizes", SIZES)
+def test_tile_edges(dc, sizes, even, sponge):
+    medium = dc.MEDIUM_PRECOMP if even else dc.MEDIUM_VPZ_VSV
+    d = (12.5, 12.5, 12.5) if even else (12.5, 10.0, 8.0)
+    coef, fields = inputs(sizes, sum(sizes))
+    sx, sy, sz = sizes
+    # receivers in neighbouring columns, several in one column, both ends of
+    # the box, and one at the source
+    xs = sorted({4, min(5, sx - 5), sx // 2, sx - 5})
+    ys = sorted({4, sy // 2, sy - 5})
+    zs = sorted({4, sz // 2, sz - 6, sz - 5} - set(range(4)))
+    rec = np.array([x + y * sx + z * sx * sy for z in zs for y in ys for x in xs])
+    src = int(rec[len(rec) // 2])
+    steps = 3
+    got, tr, en = run(dc, sizes, dc.KERNEL_FAST, medium, coef, fields, src, rec, steps, sponge, d)
+    want, _, _ = run(dc, sizes, dc.KERNEL_EXACT, medium, coef, fields, src, rec, steps, sponge, d)
+    for k in ("pp", "pc", "qp", "qc"):
+        assert rel_l2(got[k], want[k]) <= 1e-5, k
+    assert np.array_equal(tr[-1], got["pc"].reshape(-1)[rec])
+    # the energy of the last step is the sum of squares of the new fields
+    total = sum(np.sum(got[k].astype(np.float64) ** 2) for k in ("pc", "qc"))
+    assert abs(en[-1] - total) <= 1e-5 * total
