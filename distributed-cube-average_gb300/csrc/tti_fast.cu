@@ -23,8 +23,9 @@ const FastOps &ops_for(int form, int ty) {
 }
 
 // 32 x 8 tiles (two CTAs of 128 threads per SM): with 32 x 16 and one CTA of
-// 256 threads per SM nothing runs while a CTA waits at its barrier or fills
-// its queues.  DC_GB300_FAST_TY=16 selects 32 x 16.
+// 256 threads per SM nothing runs while the CTA waits at its barrier or fills
+// its queues (616^3 FP32 step 2.19 vs 2.31 ms, 872 x 872 x 616 FP16 3.79 vs
+// 4.35, 408^3 vpz/vsv 0.54 vs 0.62, 104^3 shot 2.3 vs 3.2 ms).  DC_GB300_FAST_TY=16 selects 32 x 16.
 int chosen_ty(int) {
   const char *e = std::getenv("DC_GB300_FAST_TY");
   const int v = e ? std::atoi(e) : 0;
@@ -37,22 +38,33 @@ int chosen_ty(int) {
 // planes (the 8-plane warm-up of the z queues), and the CTAs run in waves of
 // `fast_slots`, a partly filled last wave taking about as long as a full
 // one.  So the pass costs ~ ceil(tiles * chunks / slots) * (zc + 8) plane
-// sweeps; the chunk count (1..8, chunks of at least 32 planes) minimising it
-// is taken, the smaller on ties.  Measured on cubes of 200^3 to 616^3 (FP32,
-// 32 x 8 tiles, 304 slots) this choice is within 1.2 % of the fastest of
-// 1..8 chunks everywhere; one chunk per column, wherever that left the last
-// wave nearly empty, was up to 18 % slower (408^3: 0.969 vs 0.822 ms).
+// sweeps; the chunk count minimising it is taken, the smaller on ties.
+// Chunks of at least 32 planes (and at most 8) are always considered, within
+// 1.2 % of the fastest of 1..8 on cubes of 200^3 to 616^3.  Shorter ones, down
+// to kMinChunk planes, only while every SM gets one CTA at most: there the
+// step takes as long as one CTA's sweep, and the warm-up planes cost nothing
+// that was in use, not even when three simulations share the GPU.  Per step
+// alone / of three at once, FP32: 56^3 28.2 -> 7.2 / 9.6 -> 3.5 us, 72^3 19.8
+// -> 8.9 / 6.8 -> 4.6, 104^3 19.9 -> 16.1 / 10.4 -> 9.9; past one CTA per SM
+// the second figure grows (104^3 with 8 chunks: 14.3 / 11.6).
+// The energy log sums FP32 partials per column and chunk: with it on, only
+// the long chunks are considered, so that its values stay as they were.
 // DC_GB300_FAST_ZCHUNKS=<n> forces n chunks.
+constexpr long long kLongChunk = 32, kMinChunk = 4;
+
 FastShape fast_shape(const Sim *sim, long long nx, long long ny, long long nz) {
   const int ty = sim->maps_ty ? sim->maps_ty : chosen_ty(sim->coef_form);
   if (nz < 1) return FastShape{kTX, ty, 1};
   const long long tiles = std::max(1ll, (nx + kTX - 1) / kTX) * std::max(1ll, (ny + ty - 1) / ty);
   const long long slots = sim->fast_slots > 0 ? sim->fast_slots : 2 * 152;
+  const long long one_each = slots / 2;  // two CTAs fit an SM
   long long best_zc = nz, best_cost = -1;
-  for (long long c = 1; c <= 8; ++c) {
+  for (long long c = 1; c <= nz; ++c) {
     const long long zc = (nz + c - 1) / c;
-    if (c > 1 && zc < 32) break;
     const long long chunks = (nz + zc - 1) / zc;
+    if (c > 1 && (c > 8 || zc < kLongChunk) &&
+        (zc < kMinChunk || sim->d_energy || tiles * chunks > one_each))
+      break;
     const long long cost = (tiles * chunks + slots - 1) / slots * (zc + 8);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;

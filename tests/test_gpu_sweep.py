@@ -72,3 +72,27 @@ def test_tile_edges(dc, sizes, even, sponge):
     # the energy of the last step is the sum of squares of the new fields
     total = sum(np.sum(got[k].astype(np.float64) ** 2) for k in ("pc", "qc"))
     assert abs(en[-1] - total) <= 1e-5 * total
+
+
+@pytest.mark.parametrize("sizes", [(24, 24, 48), (40, 24, 13), (56, 56, 56), (72, 40, 75)])
+def test_short_chunks_change_no_bit(dc, monkeypatch, sizes):
+    """Small boxes are cut into chunks down to four planes: which CTA computes
+    a plane must not show."""
+    coef, fields = inputs(sizes, 5)
+    sx, sy, sz = sizes
+    rec = np.array([sx // 2 + (sy // 2) * sx + z * sx * sy for z in range(4, sz - 4)])
+    outs = []
+    for chunks in (None, "1", "2"):
+        if chunks:
+            monkeypatch.setenv("DC_GB300_FAST_ZCHUNKS", chunks)
+        with dc.Simulation(sizes, (12.5,) * 3, 1e-3, device=0) as sim:
+            sim.set_precomp(coef)
+            sim.set_fields(*fields)
+            sim.set_source(int(rec[3]), np.linspace(1.0, 2.0, 6))
+            sim.set_receivers(rec, 4)
+            sim.run(4)
+            sim.synchronize()
+            outs.append((sim.get_fields(), sim.traces(4)))
+    for f, tr in outs[1:]:
+        assert all(np.array_equal(f[k], outs[0][0][k]) for k in f)
+        assert np.array_equal(tr, outs[0][1])
