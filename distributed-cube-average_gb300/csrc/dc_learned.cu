@@ -107,29 +107,40 @@ __device__ __forceinline__ float gelu_grad(float a) {
   return 0.5f * (1.0f + th) + 0.5f * a * (1.0f - th * th) * du;
 }
 
-// Copies the compute parameters into shared memory.
-__device__ __forceinline__ void load_params(float *sw, const float *wc) {
-  for (int i = threadIdx.x; i < kParams; i += blockDim.x) sw[i] = wc[i];
-}
-
 // ---------------------------------------------------------------------------
 // Training: gradient of sum_i |r_i y_i - t_i|^2 over a set of samples.
-// 128 samples per CTA pass; per-sample activations and deltas live in
-// shared memory so the weight gradients are small block GEMMs over the
-// 128 samples.  `sampled` = 0: samples [0, count); 1: `count` samples
-// drawn with replacement from [0, n) by hashing `seed`.
-constexpr int kTB = 128;
-constexpr int kRow = 33;  // padded row (no bank conflicts)
-constexpr int SM_W = 0;
-constexpr int SM_XH = SM_W + kParams;
-constexpr int SM_A1 = SM_XH + kTB * kRow;   // a1, then delta1
-constexpr int SM_H1 = SM_A1 + kTB * kRow;
-constexpr int SM_A2 = SM_H1 + kTB * kRow;   // a2, then delta2
-constexpr int SM_H2 = SM_A2 + kTB * kRow;
-constexpr int SM_DY = SM_H2 + kTB * kRow;   // [kTB][2]
-constexpr int SM_DEP = SM_DY + kTB * 2;     // int
-constexpr int SM_FLOATS = SM_DEP + kTB;
-constexpr size_t kGradSmem = sizeof(float) * SM_FLOATS;
+// `sampled` = 0: samples [0, count); 1: `count` samples drawn with
+// replacement from [0, n) by hashing `seed`.
+//
+// A pass of a CTA takes 128 samples; warp w computes the hidden units
+// 4 (w / 2) .. + 3 of half of them, two neighbouring samples per lane: eight
+// chains per thread over the inputs, fed by two vector loads from shared
+// memory per input, and four chains over the samples in the weight gradients.
+// A unit's value and a pass's share of a weight's gradient stay single
+// chains, as when one thread took a whole sample (same bits).  What bounds
+// the pass is latency and the shared-memory pipe (0.1 GFLOP per 8192
+// samples): with one sample per thread each scheduler of 64 SMs had one warp
+// (44 us); a quad of units and one sample per thread, 1024 threads, issued
+// 32 k shared-memory wavefronts (24 us); a quad and four samples, 256
+// threads, left two warps per scheduler (20 us).
+constexpr int kTB = 128;           // samples per pass
+constexpr int kTT = 512;           // threads
+constexpr int kRow = kTB + 4;      // padded row: no bank conflicts along samples or units
+constexpr int kU = 4, kS = 2;      // hidden units and samples per thread
+static_assert(kIn == 32 && kHid == 32 && kTT * kU * kS == kTB * kHid && kTT == 32 * kDepths,
+              "thread tiles; one depth of b1 per warp");
+
+struct GradSmem {
+  // [unit][sample]: normalised inputs, activations and deltas
+  float xh[kIn * kRow], h1[kHid * kRow], h2[kHid * kRow], d1[kHid * kRow], d2[kHid * kRow];
+  float w1t[kIn * kHid], w2t[kHid * kHid];  // [input][unit] (forward)
+  float w2[kHid * kHid], w3[kOut * kHid];   // [unit][input] (backward)
+  float b1[kDepths * kHid], b2[kHid];
+  float dy[kOut * kTB], r[kTB];             // r: rms, 0 for silent or missing samples
+  long long idx[kTB];
+  int dep[kTB];
+  float b3[kOut];
+};
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
   z += 0x9e3779b97f4a7c15ull;
@@ -138,163 +149,255 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
   return z ^ (z >> 31);
 }
 
-__global__ void __launch_bounds__(kTB) mlp_grad_kernel(const float *__restrict__ wc,
+// a[m][i] += sum_k w[k][m] * x[k][i], k ascending: 8 chains.
+__device__ __forceinline__ void chain32(const float *w, const float *x, float a[kU][kS]) {
+#pragma unroll 8
+  for (int k = 0; k < 32; ++k) {
+    const float4 wk = *reinterpret_cast<const float4 *>(w + k * 32);
+    const float2 xk = *reinterpret_cast<const float2 *>(x + k * kRow);
+    const float wv[kU] = {wk.x, wk.y, wk.z, wk.w};
+#pragma unroll
+    for (int m = 0; m < kU; ++m) {
+      a[m][0] = fmaf(wv[m], xk.x, a[m][0]);
+      a[m][1] = fmaf(wv[m], xk.y, a[m][1]);
+    }
+  }
+}
+
+// g[o][j] += sum over the samples of d[row o][s] * x[row 16 j][s], s
+// ascending: 4 chains.
+__device__ __forceinline__ void outer128(const float *d, const float *x, float g[2][2]) {
+  float s[2][2] = {};
+#pragma unroll 4
+  for (int q = 0; q < kTB; q += 4) {
+    float4 dv[2], xv[2];
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+      dv[o] = *reinterpret_cast<const float4 *>(d + o * kRow + q);
+      xv[o] = *reinterpret_cast<const float4 *>(x + 16 * o * kRow + q);
+    }
+#pragma unroll
+    for (int o = 0; o < 2; ++o)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        s[o][j] = fmaf(dv[o].x, xv[j].x, s[o][j]);
+        s[o][j] = fmaf(dv[o].y, xv[j].y, s[o][j]);
+        s[o][j] = fmaf(dv[o].z, xv[j].z, s[o][j]);
+        s[o][j] = fmaf(dv[o].w, xv[j].w, s[o][j]);
+      }
+  }
+#pragma unroll
+  for (int o = 0; o < 2; ++o)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) g[o][j] += s[o][j];
+}
+
+__global__ void __launch_bounds__(kTT) mlp_grad_kernel(const float *__restrict__ wc,
                                                        const float *__restrict__ xs,
                                                        const float *__restrict__ ts, long long n,
                                                        long long count, unsigned long long seed,
                                                        int sampled, float *grad, double *acc) {
-  extern __shared__ float sm[];
-  float *sw = sm + SM_W;
-  float *XH = sm + SM_XH, *A1 = sm + SM_A1, *H1 = sm + SM_H1, *A2 = sm + SM_A2, *H2 = sm + SM_H2;
-  float *DY = sm + SM_DY;
-  int *DEP = reinterpret_cast<int *>(sm + SM_DEP);
-  load_params(sw, wc);
-  const int t = threadIdx.x;
-  // per-thread gradient accumulators: W1 (8), W2 (8), b1 (kDepths*kHid/128),
-  // W3 / b2 / b3 (first threads)
-  float gW1[8], gW2[8], gB1[kDepths * kHid / kTB];
-  float gW3 = 0.f, gB2 = 0.f, gB3 = 0.f;
-#pragma unroll
-  for (int m = 0; m < 8; ++m) gW1[m] = gW2[m] = 0.f;
-#pragma unroll
-  for (int m = 0; m < kDepths * kHid / kTB; ++m) gB1[m] = 0.f;
+  extern __shared__ __align__(16) unsigned char grad_smem[];
+  GradSmem &sm = *reinterpret_cast<GradSmem *>(grad_smem);
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  for (int i = t; i < kHid * kIn; i += kTT) {
+    // (transposed: the reads are scattered over the 4 KB, the stores are not)
+    const int k = i / kHid, o = i % kHid;
+    sm.w1t[i] = wc[OFF_W1 + o * kIn + k];
+    sm.w2t[i] = wc[OFF_W2 + o * kHid + k];
+    sm.w2[i] = wc[OFF_W2 + i];
+  }
+  for (int i = t; i < kDepths * kHid; i += kTT) sm.b1[i] = wc[OFF_B1 + i];
+  if (t < kOut * kHid) sm.w3[t] = wc[OFF_W3 + t];
+  if (t < kHid) sm.b2[t] = wc[OFF_B2 + t];
+  if (t < kOut) sm.b3[t] = wc[OFF_B3 + t];
+  // gradients of this thread: units go, go + 1 x inputs gk, gk + 16 of W1
+  // (warps 0-7) or W2 (8-15); unit `lane` at depth w of b1; W3 (warps 0, 1),
+  // b2 (2) and b3 (3)
+  const int go = 4 * (w & 7) + 2 * (lane >> 4), gk = lane & 15;
+  float gW[2][2] = {}, gB1 = 0.f, gX = 0.f;
   double l_err = 0.0, l_w = 0.0;
-  __syncthreads();
+  const int u0 = kU * (w >> 1), s0 = 64 * (w & 1) + kS * lane;  // this thread's units and samples
   for (long long base = static_cast<long long>(blockIdx.x) * kTB; base < count;
        base += static_cast<long long>(gridDim.x) * kTB) {
-    const long long j = base + t;
-    bool live = j < count;
-    long long i = j;
-    if (live && sampled) i = static_cast<long long>(mix64(seed ^ (static_cast<unsigned long long>(j) * 0x2545F4914F6CDD1Dull)) % static_cast<unsigned long long>(n));
-    float x[kIn];
-    int depth = 0;
-    float r = 0.f;
-    if (live) {
-      const float *row = xs + i * kStride;
+    if (t < kTB) {
+      long long i = base + t;
+      if (i >= count)
+        i = -1;
+      else if (sampled)
+        i = static_cast<long long>(mix64(seed ^ (static_cast<unsigned long long>(i) * 0x2545F4914F6CDD1Dull)) % static_cast<unsigned long long>(n));
+      sm.idx[t] = i;
+      sm.dep[t] = i >= 0 ? min(max(static_cast<int>(xs[i * kStride + kIn]), 0), kDepths - 1) : 0;
+    }
+    __syncthreads();
+    // eight sample rows per warp, transposed into [feature][sample]
+    float x[8];
 #pragma unroll
-      for (int k = 0; k < kIn; ++k) x[k] = row[k];
-      depth = min(max(static_cast<int>(row[kIn]), 0), kDepths - 1);
+    for (int q = 0; q < 8; ++q) {
+      const long long i = sm.idx[8 * w + q];
+      x[q] = i >= 0 ? xs[i * kStride + lane] : 0.0f;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q += 4)
+      *reinterpret_cast<float4 *>(sm.xh + lane * kRow + 8 * w + q) =
+          make_float4(x[q], x[q + 1], x[q + 2], x[q + 3]);
+    __syncthreads();
+    if (t < kTB) {
       float ss = 0.f;
-#pragma unroll
-      for (int k = 0; k < kIn; ++k) ss = fmaf(x[k], x[k], ss);
-      r = sqrtf(ss * (1.0f / kIn));
-      live = r > 0.f;
+#pragma unroll 8
+      for (int k = 0; k < kIn; ++k) ss = fmaf(sm.xh[k * kRow + t], sm.xh[k * kRow + t], ss);
+      sm.r[t] = sqrtf(ss * (1.0f / kIn));
     }
-    float *xh = XH + t * kRow, *a1 = A1 + t * kRow, *h1 = H1 + t * kRow;
-    float *a2 = A2 + t * kRow, *h2 = H2 + t * kRow;
-    DEP[t] = depth;
-    if (!live) {
-      for (int k = 0; k < kRow; ++k) xh[k] = a1[k] = h1[k] = a2[k] = h2[k] = 0.f;
-      DY[2 * t] = DY[2 * t + 1] = 0.f;
-    } else {
-      const float inv = 1.0f / r;
-      for (int k = 0; k < kIn; ++k) xh[k] = bf16r(x[k] * inv);
-      for (int o = 0; o < kHid; ++o) {
-        float a = sw[OFF_B1 + depth * kHid + o];
-        const float *w = sw + OFF_W1 + o * kIn;
-        for (int k = 0; k < kIn; ++k) a = fmaf(w[k], xh[k], a);
-        a1[o] = a;
-        h1[o] = bf16r(gelu(a));
+    __syncthreads();
+    bool live[kS];  // silent samples contribute nothing
+    {
+      const float2 rv = *reinterpret_cast<const float2 *>(sm.r + s0);
+      live[0] = rv.x > 0.f;
+      live[1] = rv.y > 0.f;
+      const float i0 = 1.0f / rv.x, i1 = 1.0f / rv.y;
+#pragma unroll
+      for (int m = 0; m < kU; ++m) {
+        float2 *row = reinterpret_cast<float2 *>(sm.xh + (u0 + m) * kRow + s0);
+        const float2 xv = *row;
+        *row = make_float2(live[0] ? bf16r(xv.x * i0) : 0.f, live[1] ? bf16r(xv.y * i1) : 0.f);
       }
-      for (int o = 0; o < kHid; ++o) {
-        float a = sw[OFF_B2 + o];
-        const float *w = sw + OFF_W2 + o * kHid;
-        for (int k = 0; k < kHid; ++k) a = fmaf(w[k], h1[k], a);
-        a2[o] = a;
-        h2[o] = bf16r(gelu(a));
-      }
-      float dy[kOut];
-      for (int jj = 0; jj < kOut; ++jj) {
-        float a = sw[OFF_B3 + jj];
-        const float *w = sw + OFF_W3 + jj * kHid;
-        for (int k = 0; k < kHid; ++k) a = fmaf(w[k], h2[k], a);
-        const float e = r * a - ts[i * kOut + jj];
+    }
+    __syncthreads();
+    // a layer's activations of this thread's tile, rounded, to `to`
+    auto put = [&](float *to, const float a[kU][kS]) {
+#pragma unroll
+      for (int m = 0; m < kU; ++m)
+        *reinterpret_cast<float2 *>(to + (u0 + m) * kRow + s0) = make_float2(
+            live[0] ? bf16r(gelu(a[m][0])) : 0.f, live[1] ? bf16r(gelu(a[m][1])) : 0.f);
+    };
+    float a1[kU][kS], a2[kU][kS];
+#pragma unroll
+    for (int i = 0; i < kS; ++i) {
+      const float4 bv = *reinterpret_cast<const float4 *>(sm.b1 + sm.dep[s0 + i] * kHid + u0);
+      a1[0][i] = bv.x, a1[1][i] = bv.y, a1[2][i] = bv.z, a1[3][i] = bv.w;
+    }
+    chain32(sm.w1t + u0, sm.xh + s0, a1);
+    put(sm.h1, a1);
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < kU; ++m) a2[m][0] = a2[m][1] = sm.b2[u0 + m];
+    chain32(sm.w2t + u0, sm.h1 + s0, a2);
+    put(sm.h2, a2);
+    __syncthreads();
+    if (t < kOut * kTB) {  // output j of sample s
+      const int j = t / kTB, s = t % kTB;
+      const float r = sm.r[s];
+      float d = 0.f;
+      if (r > 0.f) {
+        float a = sm.b3[j];
+#pragma unroll 8
+        for (int k = 0; k < kHid; ++k) a = fmaf(sm.w3[j * kHid + k], sm.h2[k * kRow + s], a);
+        const float e = r * a - ts[sm.idx[s] * kOut + j];
         l_err += static_cast<double>(e) * e;
-        dy[jj] = 2.0f * r * e;
-        DY[2 * t + jj] = dy[jj];
+        if (j == 0) l_w += static_cast<double>(r) * r;
+        d = 2.0f * r * e;
       }
-      l_w += static_cast<double>(r) * r;
-      // delta2 = (W3^T dy) * gelu'(a2), stored over a2
-      for (int o = 0; o < kHid; ++o) {
-        float d = 0.f;
-        for (int jj = 0; jj < kOut; ++jj) d = fmaf(sw[OFF_W3 + jj * kHid + o], dy[jj], d);
-        a2[o] = d * gelu_grad(a2[o]);
-      }
-      // delta1 = (W2^T delta2) * gelu'(a1), stored over a1
-      for (int k = 0; k < kHid; ++k) {
-        float d = 0.f;
-        for (int o = 0; o < kHid; ++o) d = fmaf(sw[OFF_W2 + o * kHid + k], a2[o], d);
-        a1[k] = d * gelu_grad(a1[k]);
+      sm.dy[t] = d;
+    }
+    __syncthreads();
+    {  // delta2 = (W3^T dy) * gelu'(a2); delta1 = (W2^T delta2) * gelu'(a1)
+      const float2 e0 = *reinterpret_cast<const float2 *>(sm.dy + s0);
+      const float2 e1 = *reinterpret_cast<const float2 *>(sm.dy + kTB + s0);
+#pragma unroll
+      for (int m = 0; m < kU; ++m) {
+        const float w30 = sm.w3[u0 + m], w31 = sm.w3[kHid + u0 + m];
+        *reinterpret_cast<float2 *>(sm.d2 + (u0 + m) * kRow + s0) = make_float2(
+            live[0] ? fmaf(w31, e1.x, fmaf(w30, e0.x, 0.f)) * gelu_grad(a2[m][0]) : 0.f,
+            live[1] ? fmaf(w31, e1.y, fmaf(w30, e0.y, 0.f)) * gelu_grad(a2[m][1]) : 0.f);
       }
     }
     __syncthreads();
-    // weight gradients: sums over the 128 samples of this pass
+    float dd[kU][kS] = {};
+    chain32(sm.w2 + u0, sm.d2 + s0, dd);
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const int e = t + kTB * m, o = e >> 5, k = e & 31;
-      float s1 = 0.f, s2 = 0.f;
-      for (int s = 0; s < kTB; ++s) {
-        s1 = fmaf(A1[s * kRow + o], XH[s * kRow + k], s1);
-        s2 = fmaf(A2[s * kRow + o], H1[s * kRow + k], s2);
-      }
-      gW1[m] += s1;
-      gW2[m] += s2;
-    }
-#pragma unroll
-    for (int m = 0; m < kDepths * kHid / kTB; ++m) {
-      const int e = t + kTB * m, dd = e / kHid, o = e % kHid;
+    for (int m = 0; m < kU; ++m)
+      *reinterpret_cast<float2 *>(sm.d1 + (u0 + m) * kRow + s0) =
+          make_float2(live[0] ? dd[m][0] * gelu_grad(a1[m][0]) : 0.f,
+                      live[1] ? dd[m][1] * gelu_grad(a1[m][1]) : 0.f);
+    __syncthreads();
+    // gradients: sums over the samples of this pass
+    outer128((w < 8 ? sm.d1 : sm.d2) + go * kRow, (w < 8 ? sm.xh : sm.h1) + gk * kRow, gW);
+    {
       float s1 = 0.f;
-      for (int s = 0; s < kTB; ++s)
-        if (DEP[s] == dd) s1 += A1[s * kRow + o];
-      gB1[m] += s1;
+#pragma unroll 4
+      for (int q = 0; q < kTB; q += 4) {
+        const int4 dq = *reinterpret_cast<const int4 *>(sm.dep + q);
+        const float4 av = *reinterpret_cast<const float4 *>(sm.d1 + lane * kRow + q);
+        if (dq.x == w) s1 += av.x;
+        if (dq.y == w) s1 += av.y;
+        if (dq.z == w) s1 += av.z;
+        if (dq.w == w) s1 += av.w;
+      }
+      gB1 += s1;
     }
-    if (t < kOut * kHid) {
-      const int jj = t / kHid, o = t % kHid;
-      float s3 = 0.f;
-      for (int s = 0; s < kTB; ++s) s3 = fmaf(DY[2 * s + jj], H2[s * kRow + o], s3);
-      gW3 += s3;
-    }
-    if (t < kHid) {
-      float s2 = 0.f;
-      for (int s = 0; s < kTB; ++s) s2 += A2[s * kRow + t];
-      gB2 += s2;
-    }
-    if (t < kOut) {
-      float s3 = 0.f;
-      for (int s = 0; s < kTB; ++s) s3 += DY[2 * s + t];
-      gB3 += s3;
+    if (w < kOut + 2) {
+      // W3: dy[j] . h2[unit]; b2: sum of delta2; b3: sum of dy
+      const float *p = w < kOut ? sm.h2 + lane * kRow
+                       : w == kOut ? sm.d2 + lane * kRow : sm.dy + (lane & (kOut - 1)) * kTB;
+      float sx = 0.f;
+#pragma unroll 4
+      for (int q = 0; q < kTB; q += 4) {
+        const float4 pv = *reinterpret_cast<const float4 *>(p + q);
+        if (w < kOut) {
+          const float4 ev = *reinterpret_cast<const float4 *>(sm.dy + w * kTB + q);
+          sx = fmaf(ev.x, pv.x, sx);
+          sx = fmaf(ev.y, pv.y, sx);
+          sx = fmaf(ev.z, pv.z, sx);
+          sx = fmaf(ev.w, pv.w, sx);
+        } else {
+          sx += pv.x;
+          sx += pv.y;
+          sx += pv.z;
+          sx += pv.w;
+        }
+      }
+      gX += sx;
     }
     __syncthreads();
   }
+  {
+    float *gw = grad + (w < 8 ? OFF_W1 : OFF_W2) + go * 32 + gk;
 #pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    atomicAdd(&grad[OFF_W1 + t + kTB * m], gW1[m]);
-    atomicAdd(&grad[OFF_W2 + t + kTB * m], gW2[m]);
+    for (int o = 0; o < 2; ++o)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) atomicAdd(&gw[o * 32 + 16 * j], gW[o][j]);
   }
+  atomicAdd(&grad[OFF_B1 + t], gB1);
+  if (w < kOut) atomicAdd(&grad[OFF_W3 + w * kHid + lane], gX);
+  if (w == kOut) atomicAdd(&grad[OFF_B2 + lane], gX);
+  if (w == kOut + 1 && lane < kOut) atomicAdd(&grad[OFF_B3 + lane], gX);
+  // loss sums (the warps that computed outputs hold them)
+  if (t < kOut * kTB) {
 #pragma unroll
-  for (int m = 0; m < kDepths * kHid / kTB; ++m) atomicAdd(&grad[OFF_B1 + t + kTB * m], gB1[m]);
-  if (t < kOut * kHid) atomicAdd(&grad[OFF_W3 + t], gW3);
-  if (t < kHid) atomicAdd(&grad[OFF_B2 + t], gB2);
-  if (t < kOut) atomicAdd(&grad[OFF_B3 + t], gB3);
-  // loss sums
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    l_err += __shfl_down_sync(0xffffffffu, l_err, off);
-    l_w += __shfl_down_sync(0xffffffffu, l_w, off);
-  }
-  if ((t & 31) == 0) {
-    atomicAdd(&acc[0], l_err);
-    atomicAdd(&acc[1], l_w);
+    for (int off = 16; off > 0; off >>= 1) {
+      l_err += __shfl_down_sync(0xffffffffu, l_err, off);
+      l_w += __shfl_down_sync(0xffffffffu, l_w, off);
+    }
+    if (lane == 0) {
+      atomicAdd(&acc[0], l_err);
+      if (t < kTB) atomicAdd(&acc[1], l_w);
+    }
   }
 }
 
 // Adam step on the FP32 master weights with the gradient of the mean loss
 // (grad / sum r^2); refreshes the compute copy (weights rounded to BF16),
-// clears the gradient and the loss sums, and records the loss.
-__global__ void mlp_adam_kernel(float *master, float *wc, float *m1, float *m2, float *grad,
-                                double *acc, float lr, float b1, float b2, float eps, int step,
-                                float *loss_hist, int hist_index) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// clears the gradient and the other step parity's loss sums, and records the
+// loss.  64 threads per CTA: the FP64 division runs at a fiftieth of the FP32
+// rate, so the parameters are spread over 42 SMs (done by the last CTA of the
+// gradient kernel instead, the step took 20 us longer).
+constexpr int kAdamT = 64;
+__global__ void __launch_bounds__(kAdamT)
+    mlp_adam_kernel(float *__restrict__ master, float *__restrict__ wc, float *__restrict__ m1,
+                    float *__restrict__ m2, float *__restrict__ grad,
+                    const double *__restrict__ acc, double *__restrict__ next_acc, float lr,
+                    float b1, float b2, float eps, int step, float *loss_hist, int hist_index) {
+  const int p = blockIdx.x * kAdamT + threadIdx.x;
   const double w = acc[1];
   if (p < kParams) {
     const float g = w > 0.0 ? static_cast<float>(grad[p] / w) : 0.0f;
@@ -309,14 +412,12 @@ __global__ void mlp_adam_kernel(float *master, float *wc, float *m1, float *m2, 
     wc[p] = is_weight(p) ? bf16r(nw) : nw;
     grad[p] = 0.0f;
   }
-  __syncthreads();
-  if (blockIdx.x == 0 && threadIdx.x == 0 && loss_hist)
-    loss_hist[hist_index] = w > 0.0 ? static_cast<float>(acc[0] / w) : 0.0f;
+  if (p == kParams) {  // a thread of the last CTA without a parameter
+    next_acc[0] = next_acc[1] = 0.0;
+    if (loss_hist) loss_hist[hist_index] = w > 0.0 ? static_cast<float>(acc[0] / w) : 0.0f;
+  }
 }
-
-__global__ void mlp_clear_acc_kernel(double *acc) {
-  if (threadIdx.x < 2) acc[threadIdx.x] = 0.0;
-}
+static_assert(kParams % kAdamT != 0, "the last CTA has a spare thread");
 
 // Compute copy of a parameter vector.
 __global__ void mlp_round_kernel(const float *master, float *wc) {
@@ -1024,7 +1125,7 @@ struct dc_gb300_mlp {
   int device = 0;
   cudaStream_t stream = nullptr;
   float *master = nullptr, *wc = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr;
-  double *acc = nullptr;
+  double *acc = nullptr;  // (sum e^2, sum r^2) per step parity
   int adam_step = 0;
 };
 
@@ -1071,7 +1172,7 @@ extern "C" int dc_gb300_mlp_create(int device, dc_gb300_mlp **out) {
       cudaMalloc(&m->master, pb) != cudaSuccess || cudaMalloc(&m->wc, pb) != cudaSuccess ||
       cudaMalloc(&m->m1, pb) != cudaSuccess || cudaMalloc(&m->m2, pb) != cudaSuccess ||
       cudaMalloc(&m->grad, pb) != cudaSuccess ||
-      cudaMalloc(&m->acc, 2 * sizeof(double)) != cudaSuccess) {
+      cudaMalloc(&m->acc, 4 * sizeof(double)) != cudaSuccess) {
     release(m);
     delete m;
     return fail(DC_GB300_ERR_NOMEM, "MLP buffers");
@@ -1155,11 +1256,12 @@ extern "C" int dc_gb300_mlp_gradient(dc_gb300_mlp *m, const float *samples, cons
   if (!m || !samples || !targets || !grad || n <= 0)
     return fail(DC_GB300_ERR_ARG, "invalid argument");
   LB_TRY(cudaSetDevice(m->device));
-  LB_TRY(cudaFuncSetAttribute(dcg::mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              static_cast<int>(dcg::kGradSmem)));
+  LB_TRY(cudaFuncSetAttribute(dcg::mlp_grad_kernel,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(sizeof(dcg::GradSmem))));
   LB_TRY(cudaMemsetAsync(m->grad, 0, sizeof(float) * dcg::kParams, m->stream));
   LB_TRY(cudaMemsetAsync(m->acc, 0, 2 * sizeof(double), m->stream));
-  dcg::mlp_grad_kernel<<<dcg::grid_for(n, dcg::kTB), dcg::kTB, dcg::kGradSmem, m->stream>>>(
+  dcg::mlp_grad_kernel<<<dcg::grid_for(n, dcg::kTB), dcg::kTT, sizeof(dcg::GradSmem), m->stream>>>(
       m->wc, samples, targets, n, n, 0ull, 0, m->grad, m->acc);
   LB_TRY(cudaGetLastError());
   double acc[2];
@@ -1181,23 +1283,24 @@ extern "C" int dc_gb300_mlp_train(dc_gb300_mlp *m, const float *samples, const f
   if (!m || !samples || !targets || n <= 0 || steps < 0 || batch < 1 || !(lr > 0))
     return fail(DC_GB300_ERR_ARG, "invalid argument");
   LB_TRY(cudaSetDevice(m->device));
-  LB_TRY(cudaFuncSetAttribute(dcg::mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              static_cast<int>(dcg::kGradSmem)));
+  LB_TRY(cudaFuncSetAttribute(dcg::mlp_grad_kernel,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(sizeof(dcg::GradSmem))));
   float *d_hist = nullptr;
   if (loss_hist && steps > 0) LB_TRY(cudaMalloc(&d_hist, sizeof(float) * steps));
   LB_TRY(cudaMemsetAsync(m->grad, 0, sizeof(float) * dcg::kParams, m->stream));
-  dcg::mlp_clear_acc_kernel<<<1, 32, 0, m->stream>>>(m->acc);
-  cudaError_t e = cudaGetLastError();
+  LB_TRY(cudaMemsetAsync(m->acc, 0, 4 * sizeof(double), m->stream));
+  cudaError_t e = cudaSuccess;
   const int blocks = dcg::grid_for(batch, dcg::kTB);
   for (int s = 0; s < steps && e == cudaSuccess; ++s) {
-    dcg::mlp_grad_kernel<<<blocks, dcg::kTB, dcg::kGradSmem, m->stream>>>(
+    double *acc = m->acc + 2 * (s & 1), *next = m->acc + 2 * (1 - (s & 1));
+    dcg::mlp_grad_kernel<<<blocks, dcg::kTT, sizeof(dcg::GradSmem), m->stream>>>(
         m->wc, samples, targets, n, batch, seed + 0x9E3779B97F4A7C15ull * (m->adam_step + 1), 1,
-        m->grad, m->acc);
+        m->grad, acc);
     ++m->adam_step;
-    dcg::mlp_adam_kernel<<<(dcg::kParams + 255) / 256, 256, 0, m->stream>>>(
-        m->master, m->wc, m->m1, m->m2, m->grad, m->acc, lr, 0.9f, 0.999f, 1e-8f, m->adam_step,
-        d_hist, s);
-    dcg::mlp_clear_acc_kernel<<<1, 32, 0, m->stream>>>(m->acc);
+    dcg::mlp_adam_kernel<<<(dcg::kParams + dcg::kAdamT - 1) / dcg::kAdamT, dcg::kAdamT, 0,
+                           m->stream>>>(m->master, m->wc, m->m1, m->m2, m->grad, acc, next, lr,
+                                        0.9f, 0.999f, 1e-8f, m->adam_step, d_hist, s);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && d_hist)
