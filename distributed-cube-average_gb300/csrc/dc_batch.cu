@@ -82,8 +82,8 @@ struct Batch {
   // launches in the step graph (stencil, then its layer), so one half's
   // network overlaps the other half's stencil.
   struct LbBranch {
-    int4 *d_lines = nullptr;   // face lines (meta bits 8..31: the shot)
-    int4 *d_edge = nullptr;    // edge cells
+    int4 *d_lines = nullptr;   // face lines and edge cells (layer_tables)
+    int4 *d_edge = nullptr;
     float2 *d_corr = nullptr;  // edge-cell corrections
     long long nl = 0, ne = 0;
   } lb[2];
@@ -832,17 +832,12 @@ extern "C" int dc_gb300_batch_set_learned_layer(dc_gb300_batch *h, const dc_gb30
     const dcg::BShot &s = b->shots[k];
     if (s.cfg.sx < 2 * layer + 16 || s.cfg.sy < 2 * layer + 16 || s.cfg.sz < 2 * layer + 16)
       return fail(DC_GB300_ERR_ARG, "every shot's interior must keep at least 8 cells per axis");
-    const dcg::LayerPlan plan = dcg::layer_plan(s.cfg.sx, s.cfg.sy, s.cfg.sz, layer);
-    for (int4 v : plan.lines) {
-      v.w |= static_cast<int>(k) << 8;
-      lines[br].push_back(v);
-    }
-    for (int4 v : plan.edge) {
-      v.w |= static_cast<int>(k) << 8;
-      edge[br].push_back(v);
-    }
+    const dcg::LayerTables plan = dcg::layer_tables(s.cfg.sx, s.cfg.sy, s.cfg.sz, s.pitch, layer,
+                                                    static_cast<int>(k));
+    lines[br].insert(lines[br].end(), plan.lines.begin(), plan.lines.end());
+    edge[br].insert(edge[br].end(), plan.edge.begin(), plan.edge.end());
     total += static_cast<long long>(dcg::layer_cells(s.cfg.sx, s.cfg.sy, s.cfg.sz, layer).size());
-    tab.push_back(dcg::LbShot{{s.pq[0], s.pq[1]}, s.pitch, s.plane});
+    tab.push_back(dcg::LbShot{{s.pq[0], s.pq[1]}});
   }
   for (int br = 0; br < b->nbranch; ++br) {
     Batch::LbBranch &l = b->lb[br];

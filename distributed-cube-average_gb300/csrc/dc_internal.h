@@ -355,18 +355,23 @@ cudaError_t launch_lb_sample(cudaStream_t st, const int4 *cells, long long n, co
                              const float2 *cur, long long pitch, long long plane,
                              const float2 *wide, long long wpitch, long long wplane,
                              const int off[3], float *xs, float *ts);
-// Learned layer over a batch: cells carry their shot in meta bits 8..31.
-struct LbShot {
-  float2 *pq[2];              // the shot's pair buffers
-  long long pitch, plane;
+// The layer plan as the in-step kernels read it: {offset low, offset high,
+// inward stride, code}, offset and stride in pairs of the box's buffers; code =
+// depth of an edge cell (0 for a line) | shot << 8.
+struct LayerTables {
+  std::vector<int4> lines, edge;
 };
-cudaError_t launch_lb_batch_step(cudaStream_t st, const float *params, const int4 *cells,
-                                 long long n, const LbShot *shots, int cur_buf, float2 *corr);
-// The in-step correction through the face lines and the edge cells.
-// Bit-identical to launch_lb_step over all corrected cells.
+LayerTables layer_tables(long long sx, long long sy, long long sz, long long pitch, int layer,
+                         int shot);
+// A shot's pair buffers (learned layer over a batch).
+struct LbShot {
+  float2 *pq[2];
+};
+// The in-step correction through the face lines and the edge cells
+// (layer_tables).  Bit-identical to launch_lb_step over all corrected cells.
 cudaError_t launch_lb_fused(cudaStream_t st, const float *params, int layer, const int4 *lines,
                             long long nl, const int4 *edge, long long ne, float2 *nw,
-                            const float2 *cur, long long pitch, long long plane, float2 *corr);
+                            const float2 *cur, float2 *corr);
 cudaError_t launch_lb_batch_fused(cudaStream_t st, const float *params, int layer,
                                   const int4 *lines, long long nl, const int4 *edge, long long ne,
                                   const LbShot *shots, int cur_buf, float2 *corr);

@@ -548,15 +548,59 @@ struct CellSrc {  // the layer cells of one simulation
   }
 };
 
-struct BatchCellSrc {  // the layer cells of every shot of a batch
-  const int4 *cells;
+// Entries of the in-step tables (face lines and edge cells): {offset low,
+// offset high, inward stride, code}, made by layer_tables; code = depth of an
+// edge cell | shot << 8.  (With coordinates the kernels spent a sixth of their
+// instructions on 64-bit index products.)
+__device__ __forceinline__ long long entry_offset(const int4 e) {
+  return static_cast<long long>(static_cast<uint32_t>(e.x)) | static_cast<long long>(e.y) << 32;
+}
+
+struct LinePtr {
+  float2 *nw;         // the entry's (outermost) cell in the new field
+  const float2 *cur;  // ... in the current field
+  int step;           // inward stride
+};
+
+struct SimEntries {  // table of one simulation
+  const int4 *table;
+  float2 *nw;
+  const float2 *cur;
+  __device__ __forceinline__ LinePtr at(const int4 e) const {
+    const long long o = entry_offset(e);
+    return LinePtr{nw + o, cur + o, e.z};
+  }
+};
+
+struct BatchEntries {  // table over the shots of a batch
+  const int4 *table;
   const LbShot *shots;
   int cur_buf;
-  __device__ __forceinline__ int load(long long r, int t, float f[8]) const {
-    int4 c = cells[r];
-    const LbShot &sh = shots[c.w >> 8];
-    c.w &= 0xff;
-    return load_cell(c, sh.pq[1 - cur_buf], sh.pq[cur_buf], sh.pitch, sh.plane, t, f, nullptr);
+  __device__ __forceinline__ LinePtr at(const int4 e) const {
+    const LbShot &sh = shots[e.w >> 8];
+    const long long o = entry_offset(e);
+    return LinePtr{sh.pq[1 - cur_buf] + o, sh.pq[cur_buf] + o, e.z};
+  }
+};
+
+template <class Entries>
+struct EdgeSrc {  // edge cells: features of the cell's window
+  Entries t;
+  __device__ __forceinline__ int load(long long r, int q, float f[8]) const {
+    const int4 e = t.table[r];
+    const LinePtr p = t.at(e);
+    const long long o = static_cast<long long>(2 * q) * p.step;
+    const float2 *n = p.nw + o, *c = p.cur + o;
+    const float2 a0 = n[0], a1 = n[p.step], b0 = c[0], b1 = c[p.step];
+    f[0] = a0.x;
+    f[1] = a1.x;
+    f[2] = a0.y;
+    f[3] = a1.y;
+    f[4] = b0.x;
+    f[5] = b1.x;
+    f[6] = b0.y;
+    f[7] = b1.y;
+    return e.w & 0xff;
   }
 };
 
@@ -664,6 +708,86 @@ __device__ __forceinline__ bool net16(const NetSmem &sm, const float f0[8], cons
   return true;
 }
 
+// The network over the 32 rows of two tiles: lane (g, t) brings the features
+// f[q] of rows g (q = 0), g + 8 (1) of the first tile and g (2), g + 8 (3) of
+// the second, all with this lane's first bias b1 (pairs of units 8 nt + 2t).
+// Every weight fragment is loaded once for both tiles.  Returns a bit per
+// tile that is not silent (0: nothing was computed); the lanes with t == 0
+// then hold the corrections rr[q] * y[q].  Each tile's arithmetic is net16's.
+__device__ __forceinline__ int net32(const NetSmem &sm, const float f[4][8], const float2 b1[4],
+                                     const float2 b2[4], float rr[4], float2 y[4]) {
+  const int lane = threadIdx.x & 31, t = lane & 3;
+  float inv[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s = fmaf(f[q][k], f[q][k], s);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    rr[q] = s;
+  }
+  const int live = (__all_sync(0xffffffffu, rr[0] == 0.f && rr[1] == 0.f) ? 0 : 1) |
+                   (__all_sync(0xffffffffu, rr[2] == 0.f && rr[3] == 0.f) ? 0 : 2);
+  if (!live) return 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    rr[q] = sqrtf(rr[q] * (1.0f / kIn));
+    inv[q] = rr[q] > 0.f ? 1.0f / rr[q] : 0.f;
+  }
+  uint32_t a[2][2][4];  // [tile][k chunk]
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk) {
+      const float *f0 = f[2 * m], *f1 = f[2 * m + 1];
+      const float i0 = inv[2 * m], i1 = inv[2 * m + 1];
+      a[m][kk][0] = pack_bf16(f0[4 * kk] * i0, f0[4 * kk + 1] * i0);
+      a[m][kk][1] = pack_bf16(f1[4 * kk] * i1, f1[4 * kk + 1] * i1);
+      a[m][kk][2] = pack_bf16(f0[4 * kk + 2] * i0, f0[4 * kk + 3] * i0);
+      a[m][kk][3] = pack_bf16(f1[4 * kk + 2] * i1, f1[4 * kk + 3] * i1);
+    }
+  float acc[2][4][4];
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    const uint2 w0 = sm.w1[0][nt][lane], w1 = sm.w1[1][nt][lane];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      acc[m][nt][0] = acc[m][nt][2] = b1[nt].x;
+      acc[m][nt][1] = acc[m][nt][3] = b1[nt].y;
+      mma_bf16(acc[m][nt], a[m][0], w0.x, w0.y);
+      mma_bf16(acc[m][nt], a[m][1], w1.x, w1.y);
+    }
+  }
+  gelu_to_a(acc[0], a[0]);
+  gelu_to_a(acc[1], a[1]);
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    const uint2 w0 = sm.w2[0][nt][lane], w1 = sm.w2[1][nt][lane];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      acc[m][nt][0] = acc[m][nt][2] = b2[nt].x;
+      acc[m][nt][1] = acc[m][nt][3] = b2[nt].y;
+      mma_bf16(acc[m][nt], a[m][0], w0.x, w0.y);
+      mma_bf16(acc[m][nt], a[m][1], w1.x, w1.y);
+    }
+  }
+  gelu_to_a(acc[0], a[0]);
+  gelu_to_a(acc[1], a[1]);
+  const uint2 w0 = sm.w3[0][lane], w1 = sm.w3[1][lane];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    float o[4];
+    o[0] = o[2] = t == 0 ? sm.b3[0] : 0.f;
+    o[1] = o[3] = t == 0 ? sm.b3[1] : 0.f;
+    mma_bf16(o, a[m][0], w0.x, w0.y);
+    mma_bf16(o, a[m][1], w1.x, w1.y);
+    y[2 * m] = make_float2(o[0], o[1]);
+    y[2 * m + 1] = make_float2(o[2], o[3]);
+  }
+  return live;
+}
+
 // One correction per cell or sample row, written to out (zeros for silent
 // rows): the training-side and recorded-rollout evaluation.
 template <class Src>
@@ -704,55 +828,27 @@ __global__ void __launch_bounds__(128, 8) lb_tc_kernel(const float *__restrict__
 // corrected cells of one boundary normal (outermost first) whose tangential
 // coordinates lie far enough inside the other two axes' interiors that no
 // other line's cell is in its windows and no other cell's window reaches it
-// (layer_plan below); its kLine windows span kLineCells distinct cells.  One
-// warp takes 4 lines -- the 16 rows of one MMA pass: it gathers the 4 x
-// kLineCells cells of both time levels once into shared memory, evaluates
-// the network and adds each correction in place.  Every value a warp reads
-// was read before it writes, and no other warp touches its lines, so the
-// result is bit-identical to the two-pass form (lb_tc_kernel then
-// lb_add_kernel) while reading each cell once instead of up to 8 times.
+// (layer_plan below); its kLine windows span kLineCells distinct cells.  A
+// warp takes 16 lines, four of them to the 16 rows of an MMA tile: it gathers
+// the 16 x kLineCells cells of both time levels once into shared memory,
+// evaluates the network over two tiles at a time and stores the corrected
+// cells.  Every value a warp reads was read before it writes, and no other
+// warp touches its lines, so the result is bit-identical to the two-pass form
+// (lb_tc_kernel then the add) while reading each cell once instead of up to
+// 8 times.
+//
+// What bounds it: the shared-memory pipe, then the special-function pipe (32
+// tanh per tile).  Sixteen lines per warp, because neighbours in the table
+// are neighbours in x on four of the six faces: one gather instruction brings
+// two 128-byte runs (with four lines eight 32-byte ones).  [line][cell] in
+// shared memory and weight fragments shared by two tiles issue 60 wavefronts
+// per tile where [cell][line] and a tile at a time issued 130 (82 % of the
+// pipe); that costs registers, so four CTAs per SM instead of eight.
 constexpr int kLine = kCorrected;               // corrected cells per line
 constexpr int kLineCells = kLine + kWin - 1;    // cells the line's windows span
-constexpr int kLineWarp = 16 / kLine;           // lines per warp pass
-constexpr int kGather = 2 * kLineCells * kLineWarp;  // float2 loads per warp pass
-constexpr int kGatherPerLane = (kGather + 31) / 32;
-static_assert(16 % kLine == 0 && 32 % kLineWarp == 0, "line packing of the MMA rows");
-
-struct LinePtr {
-  float2 *nw;         // the line's outermost cell in the new field
-  const float2 *cur;  // ... in the current field
-  long long step;     // inward stride
-};
-
-__device__ __forceinline__ long long inward_step(int code, long long pitch, long long plane) {
-  const int axis = code & 3, side = (code >> 2) & 1;
-  const long long stride = axis == 0 ? 1 : axis == 1 ? pitch : plane;
-  return side ? -stride : stride;
-}
-
-struct LineSrc {  // the face lines of one simulation
-  const int4 *lines;
-  float2 *nw;
-  const float2 *cur;
-  long long pitch, plane;
-  __device__ __forceinline__ LinePtr at(const int4 c) const {
-    const long long g = static_cast<long long>(c.z) * plane + static_cast<long long>(c.y) * pitch + c.x;
-    return LinePtr{nw + g, cur + g, inward_step(c.w, pitch, plane)};
-  }
-};
-
-struct BatchLineSrc {  // the face lines of every shot of a batch
-  const int4 *lines;
-  const LbShot *shots;
-  int cur_buf;
-  __device__ __forceinline__ LinePtr at(const int4 c) const {
-    const LbShot &sh = shots[c.w >> 8];
-    const long long g = static_cast<long long>(c.z) * sh.plane +
-                        static_cast<long long>(c.y) * sh.pitch + c.x;
-    return LinePtr{sh.pq[1 - cur_buf] + g, sh.pq[cur_buf] + g,
-                   inward_step(c.w, sh.pitch, sh.plane)};
-  }
-};
+constexpr int kLineWarp = 16;                   // lines per warp pass
+constexpr int kLineCtas = 4;                    // CTAs per SM
+static_assert(kLine == 4 && kLineWarp == 16, "four lines to a 16-row tile, four tiles");
 
 // Asynchronous 8-byte copy global -> shared (zero fill when !valid; gsrc
 // must still be a mapped address).
@@ -769,124 +865,113 @@ __device__ __forceinline__ void cp_async_wait0() {
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Each warp keeps one pass's copies in flight while the network runs on
-// the previous one: at the top of pass p it waits for the group that
-// brought pass p's cells and pass p+1's line entries, then queues pass
-// p+1's cells (addresses from those entries) and pass p+2's entries.
-// Cells and entries are double-buffered in shared memory; nothing waits on
-// a global load issued in the same pass.
-template <class Src>
-__global__ void __launch_bounds__(128, 8) lb_line_kernel(const float *__restrict__ wc, Src src,
-                                                         long long nlines, int layer) {
+// Each warp keeps one pass's copies in flight while the network runs on the
+// previous one: at the top of pass p it waits for pass p's cells and queues
+// pass p + 1's, whose addresses it worked out during pass p - 1 from entries
+// loaded during pass p - 2.  Nothing waits on a global load issued in the
+// same pass.
+template <class Entries>
+__global__ void __launch_bounds__(128, kLineCtas)
+    lb_line_kernel(const float *__restrict__ wc, Entries src, long long nlines, int layer) {
   __shared__ NetSmem sm;
-  // per warp and buffer: [field][cell][line] (field 0 = new, 1 = current),
-  // the lines' table entries, and their new-field pointers and strides
-  __shared__ __align__(16) float2 sl[4][2][2][kLineCells][kLineWarp];
-  __shared__ __align__(16) int4 sent[4][2][kLineWarp];
-  __shared__ float2 *snw[4][2][kLineWarp];
-  __shared__ long long sst[4][2][kLineWarp];
+  // per warp and buffer: [field][line][cell] (field 0 = new, 1 = current)
+  __shared__ __align__(16) float2 sl[4][2][2][kLineWarp][kLineCells];
   stage_net(wc, sm);
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = threadIdx.x >> 5;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-  const long long stride = nwarps * kLineWarp;
-  // rows g and g + 8: position j of lines la and lb
-  const int j = g % kLine, la = g / kLine, lb = la + 8 / kLine;
+  const long long stride = ((static_cast<long long>(gridDim.x) * blockDim.x) >> 5) * kLineWarp;
+  // rows g and g + 8 of a tile: position j of lines g / 4 and g / 4 + 2
+  const int j = g % kLine;
   const int depth = layer - 1 - j;
-  const int ml = lane % kLineWarp;  // the line this lane copies (32 is a multiple of 4)
-  const float2 *dummy = reinterpret_cast<const float2 *>(wc);
-  // queues the table entries of the pass at `base` into entry buffer `buf`
-  auto fetch_entries = [&](long long base, int buf) {
-    if (lane < kLineWarp) {
-      const bool v = base + lane < nlines;
-      const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(&sent[w][buf][lane]));
-      const void *from = v ? static_cast<const void *>(src.lines + base + lane)
-                           : static_cast<const void *>(wc);
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(from),
-                   "r"(v ? 16 : 0)
-                   : "memory");
-    }
-  };
-  // queues the cells of the pass at `base` (entries in buffer `buf`) into
-  // cell buffer `buf`
-  auto fetch_cells = [&](long long base, int buf) {
-    const bool mv = base + ml < nlines;
-    LinePtr lp{nullptr, nullptr, 0};
-    if (mv) lp = src.at(sent[w][buf][ml]);
-    if (lane < kLineWarp) {
-      snw[w][buf][lane] = lp.nw;
-      sst[w][buf][lane] = lp.step;
-    }
+  const int ml = lane % kLineWarp, half = lane / kLineWarp;  // line and parity of cells copied
+  float2 b1[4], b2[4];
 #pragma unroll
-    for (int k = 0; k < kGatherPerLane; ++k) {
-      const int i = lane + 32 * k;
-      const int fld = i / (kLineCells * kLineWarp), c = (i / kLineWarp) % kLineCells;
-      if (i < kGather)
-        cp_async8(&sl[w][buf][fld][c][ml], mv ? (fld ? lp.cur : lp.nw) + c * lp.step : dummy,
-                  mv);
+  for (int nt = 0; nt < 4; ++nt) {
+    const int c = nt * 8 + 2 * t;
+    b1[nt] = make_float2(sm.b1[depth * kHid + c], sm.b1[depth * kHid + c + 1]);
+    b2[nt] = make_float2(sm.b2[c], sm.b2[c + 1]);
+  }
+  auto entry = [&](long long base) {  // (code -1: no line)
+    return base + ml < nlines ? src.table[base + ml] : make_int4(0, 0, 0, -1);
+  };
+  auto pointers = [&](const int4 e) {
+    return e.w >= 0 ? src.at(e) : LinePtr{nullptr, nullptr, 0};
+  };
+  auto fetch = [&](const LinePtr p, int buf) {
+    const bool v = p.nw != nullptr;
+    const float2 *dummy = reinterpret_cast<const float2 *>(wc);
+    const float2 *n = (v ? p.nw : dummy) + half * p.step, *c = (v ? p.cur : dummy) + half * p.step;
+    const long long two = 2ll * p.step;
+#pragma unroll
+    for (int k = 0; k < kLineCells; k += 2) {
+      if (k + half < kLineCells) {
+        cp_async8(&sl[w][buf][0][ml][k + half], n, v);
+        cp_async8(&sl[w][buf][1][ml][k + half], c, v);
+      }
+      n += two;
+      c += two;
     }
   };
   long long base = warp * kLineWarp;
-  if (base < nlines) {
-    fetch_entries(base, 0);
-    cp_async_commit();
-    cp_async_wait0();
-    __syncwarp();
-    fetch_cells(base, 0);
-    fetch_entries(base + stride, 1);
-  }
+  if (base >= nlines) return;  // (no CTA barrier below)
+  LinePtr now = pointers(entry(base)), next = pointers(entry(base + stride));
+  int4 after = entry(base + 2 * stride);
+  fetch(now, 0);
   cp_async_commit();
   for (int buf = 0; base < nlines; base += stride, buf ^= 1) {
-    cp_async_wait0();  // this pass's cells and the next pass's entries have landed
-    __syncwarp();
-    if (base + stride < nlines) {
-      fetch_cells(base + stride, buf ^ 1);
-      fetch_entries(base + 2 * stride, buf);
-    }
+    cp_async_wait0();  // this pass's cells have landed
+    __syncwarp();      // every lane has read the other buffer
+    if (base + stride < nlines) fetch(next, buf ^ 1);
     cp_async_commit();
-    float2(*ls)[kLineCells][kLineWarp] = sl[w][buf];
-    float f0[8], f1[8];
-    {
-      const int c0 = j + 2 * t, c1 = c0 + 1;
-      const float2 a0 = ls[0][c0][la], a1 = ls[0][c1][la];
-      const float2 b0 = ls[1][c0][la], b1 = ls[1][c1][la];
-      f0[0] = a0.x, f0[1] = a1.x, f0[2] = a0.y, f0[3] = a1.y;
-      f0[4] = b0.x, f0[5] = b1.x, f0[6] = b0.y, f0[7] = b1.y;
-      const float2 e0 = ls[0][c0][lb], e1 = ls[0][c1][lb];
-      const float2 h0 = ls[1][c0][lb], h1 = ls[1][c1][lb];
-      f1[0] = e0.x, f1[1] = e1.x, f1[2] = e0.y, f1[3] = e1.y;
-      f1[4] = h0.x, f1[5] = h1.x, f1[6] = h0.y, f1[7] = h1.y;
-    }
-    float rr0 = 0.f, rr1 = 0.f, y[4];
-    if (net16(sm, f0, f1, depth, depth, rr0, rr1, y) && t == 0) {
-      // new value = stencil output + correction, rounded as the two-pass form
-      if (base + la < nlines) {
-        const float2 v = ls[0][j][la];
-        snw[w][buf][la][j * sst[w][buf][la]] = make_float2(
-            __fadd_rn(v.x, __fmul_rn(rr0, y[0])), __fadd_rn(v.y, __fmul_rn(rr0, y[1])));
+    const LinePtr third = pointers(after);
+    after = entry(base + 3 * stride);
+    float2(*ls)[kLineWarp][kLineCells] = sl[w][buf];
+    int live = 0;  // a bit per tile
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      const int l0 = 8 * h + g / kLine, c0 = j + 2 * t;
+      float f[4][8], rr[4];
+      float2 y[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float2 *n = &ls[0][l0 + 2 * q][c0], *c = &ls[1][l0 + 2 * q][c0];
+        const float2 a0 = n[0], a1 = n[1], e0 = c[0], e1 = c[1];
+        f[q][0] = a0.x, f[q][1] = a1.x, f[q][2] = a0.y, f[q][3] = a1.y;
+        f[q][4] = e0.x, f[q][5] = e1.x, f[q][6] = e0.y, f[q][7] = e1.y;
       }
-      if (base + lb < nlines) {
-        const float2 v = ls[0][j][lb];
-        snw[w][buf][lb][j * sst[w][buf][lb]] = make_float2(
-            __fadd_rn(v.x, __fmul_rn(rr1, y[2])), __fadd_rn(v.y, __fmul_rn(rr1, y[3])));
+      const int lv = net32(sm, f, b1, b2, rr, y);
+      live |= lv << (2 * h);
+      __syncwarp();  // every lane has its features
+      if (t == 0) {
+        // new value = stencil output + correction, rounded as the two-pass
+        // form
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (lv & (1 << (q / 2))) {
+            float2 &v = ls[0][l0 + 2 * q][j];
+            v = make_float2(__fadd_rn(v.x, __fmul_rn(rr[q], y[q].x)),
+                            __fadd_rn(v.y, __fmul_rn(rr[q], y[q].y)));
+          }
       }
     }
-    __syncwarp();  // the pass after next overwrites this buffer
+    __syncwarp();
+    // the corrected cells of the tiles that were evaluated
+    if (now.nw && (live >> (ml / kLine)) & 1)
+#pragma unroll
+      for (int k = 0; k < kLine; k += 2)
+        now.nw[static_cast<long long>(k + half) * now.step] = ls[0][ml][k + half];
+    now = next;
+    next = third;
   }
 }
 
-__global__ void lb_add_batch_kernel(const int4 *__restrict__ cells, long long n,
-                                    const LbShot *__restrict__ shots, int cur_buf,
-                                    const float2 *__restrict__ corr) {
+template <class Entries>
+__global__ void lb_add_edge_kernel(Entries src, long long n, const float2 *__restrict__ corr) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int4 c = cells[i];
-    const LbShot sh = shots[c.w >> 8];
-    float2 *nw = sh.pq[1 - cur_buf];
-    const long long g = static_cast<long long>(c.z) * sh.plane +
-                        static_cast<long long>(c.y) * sh.pitch + c.x;
-    const float2 d = corr[i], v = nw[g];
-    nw[g] = make_float2(v.x + d.x, v.y + d.y);
+    float2 *p = src.at(src.table[i]).nw;
+    const float2 d = corr[i], v = *p;
+    *p = make_float2(v.x + d.x, v.y + d.y);
   }
 }
 
@@ -957,10 +1042,12 @@ __global__ void crop_kernel(float2 *dst, long long sx, long long sy, long long s
   }
 }
 
-// The face-line pass: at most one wave of its 8 CTAs per SM (each stages
-// the weights once and loops over its passes).
+// The face-line pass: at most one wave of its CTAs (each stages the weights
+// once and loops over its passes; four warps of kLineWarp lines).
 int line_grid(long long nl) {
-  return static_cast<int>(std::max<long long>(1, std::min<long long>((nl + 15) / 16, 152 * 8)));
+  const long long per = 4 * kLineWarp;
+  return static_cast<int>(
+      std::max<long long>(1, std::min<long long>((nl + per - 1) / per, 152 * kLineCtas)));
 }
 
 int grid_for(long long n, int per_block) {
@@ -1019,16 +1106,6 @@ cudaError_t launch_lb_step(cudaStream_t st, const float *wc, const int4 *cells, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_lb_batch_step(cudaStream_t st, const float *wc, const int4 *cells,
-                                 long long n, const LbShot *shots, int cur_buf, float2 *corr) {
-  lb_tc_kernel<BatchCellSrc><<<grid_for(n, 64), 128, 0, st>>>(
-      wc, BatchCellSrc{cells, shots, cur_buf}, n, corr);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  lb_add_batch_kernel<<<grid_for(n, 256), 256, 0, st>>>(cells, n, shots, cur_buf, corr);
-  return cudaGetLastError();
-}
-
 // Splits the corrected cells into face lines (entries for the outermost
 // cell, meta = axis | side << 2) and the remaining edge cells (layer_cells
 // entries).  The windows of the least deep corrected cells reach m cells
@@ -1064,30 +1141,59 @@ LayerPlan layer_plan(long long sx, long long sy, long long sz, int layer) {
   return plan;
 }
 
-cudaError_t launch_lb_fused(cudaStream_t st, const float *wc, int layer, const int4 *lines,
-                            long long nl, const int4 *edge, long long ne, float2 *nw,
-                            const float2 *cur, long long pitch, long long plane, float2 *corr) {
+LayerTables layer_tables(long long sx, long long sy, long long sz, long long pitch, int layer,
+                         int shot) {
+  const LayerPlan plan = layer_plan(sx, sy, sz, layer);
+  const long long plane = pitch * sy;
+  auto pack = [&](const int4 &c, int code) {
+    const long long off = c.z * plane + c.y * pitch + c.x;
+    const int axis = c.w & 3, side = (c.w >> 2) & 1;
+    const long long stride = axis == 0 ? 1 : axis == 1 ? pitch : plane;
+    return make_int4(static_cast<int>(off & 0xffffffffll), static_cast<int>(off >> 32),
+                     static_cast<int>(side ? -stride : stride), code | shot << 8);
+  };
+  LayerTables out;
+  out.lines.reserve(plan.lines.size());
+  out.edge.reserve(plan.edge.size());
+  for (const int4 &c : plan.lines) out.lines.push_back(pack(c, 0));
+  for (const int4 &c : plan.edge) out.edge.push_back(pack(c, (c.w >> 3) & 31));
+  return out;
+}
+
+namespace {
+
+// The face lines in place, then the edge cells through `corr`.
+template <class Entries>
+cudaError_t launch_entries(cudaStream_t st, const float *wc, int layer, Entries lines,
+                           long long nl, Entries edge, long long ne, float2 *corr) {
   if (nl > 0) {
-    lb_line_kernel<LineSrc><<<line_grid(nl), 128, 0, st>>>(
-        wc, LineSrc{lines, nw, cur, pitch, plane}, nl, layer);
+    lb_line_kernel<Entries><<<line_grid(nl), 128, 0, st>>>(wc, lines, nl, layer);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  if (ne > 0) return launch_lb_step(st, wc, edge, ne, nw, cur, pitch, plane, corr, nullptr);
-  return cudaSuccess;
+  if (ne <= 0) return cudaSuccess;
+  lb_tc_kernel<EdgeSrc<Entries>><<<grid_for(ne, 64), 128, 0, st>>>(wc, EdgeSrc<Entries>{edge}, ne,
+                                                                   corr);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  lb_add_edge_kernel<Entries><<<grid_for(ne, 256), 256, 0, st>>>(edge, ne, corr);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_lb_fused(cudaStream_t st, const float *wc, int layer, const int4 *lines,
+                            long long nl, const int4 *edge, long long ne, float2 *nw,
+                            const float2 *cur, float2 *corr) {
+  return launch_entries(st, wc, layer, SimEntries{lines, nw, cur}, nl, SimEntries{edge, nw, cur},
+                        ne, corr);
 }
 
 cudaError_t launch_lb_batch_fused(cudaStream_t st, const float *wc, int layer, const int4 *lines,
                                   long long nl, const int4 *edge, long long ne,
                                   const LbShot *shots, int cur_buf, float2 *corr) {
-  if (nl > 0) {
-    lb_line_kernel<BatchLineSrc><<<line_grid(nl), 128, 0, st>>>(
-        wc, BatchLineSrc{lines, shots, cur_buf}, nl, layer);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  if (ne > 0) return launch_lb_batch_step(st, wc, edge, ne, shots, cur_buf, corr);
-  return cudaSuccess;
+  return launch_entries(st, wc, layer, BatchEntries{lines, shots, cur_buf}, nl,
+                        BatchEntries{edge, shots, cur_buf}, ne, corr);
 }
 
 cudaError_t launch_lb_sample(cudaStream_t st, const int4 *cells, long long n, const float2 *nw,

@@ -316,8 +316,7 @@ cudaError_t queue_step(Sim *s, int j) {
     } else {
       s->launches += launches_per_step(s) - 1;
       e = launch_lb_fused(s->stream, s->lb_params, s->lb_layer, s->d_lb_lines, s->lb_lines,
-                          s->d_lb_edge, s->lb_edge, s->pq[prev], s->pq[cur], s->pitch,
-                          s->plane, s->d_lb_corr);
+                          s->d_lb_edge, s->lb_edge, s->pq[prev], s->pq[cur], s->d_lb_corr);
     }
     if (e != cudaSuccess) return e;
   }
@@ -1058,7 +1057,7 @@ extern "C" int dc_gb300_set_learned_layer(dc_gb300_sim *h, const dc_gb300_mlp *m
   free_layer(s);
   if (layer == 0) return DC_GB300_OK;
   const std::vector<int4> cells = layer_cells(s->sx, s->sy, s->sz, layer);
-  const LayerPlan plan = layer_plan(s->sx, s->sy, s->sz, layer);
+  const LayerTables plan = layer_tables(s->sx, s->sy, s->sz, s->pitch, layer, 0);
   const long long n = static_cast<long long>(cells.size());
   const long long nl = static_cast<long long>(plan.lines.size());
   const long long ne = static_cast<long long>(plan.edge.size());
