@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -103,6 +104,9 @@ struct StepParams {
   float *traces;
   int nrec, trace_cap, col_stride;
   int *err;
+  // 1: the pass touches nothing that the pass launched just before it writes
+  // (another box of the same step): it may run beside it
+  int beside;
   // position of the box's point (0, 0, 0) in the medium's arrays (the
   // batched form crops shots out of one shared medium; 0 otherwise)
   int mox, moy, moz;
@@ -170,6 +174,11 @@ struct Sim {
   int *d_err = nullptr;
   long long launches = 0;
   int config_version = 0;
+  // boxes {x0, y0, z0, x1, y1, z1} of the propagate calls since any other call,
+  // and the roles (pp, pc) they ran with
+  std::vector<std::array<long long, 6>> boxes;
+  const float *box_pp = nullptr, *box_pc = nullptr;
+  bool stream_shared = false;  // the caller has been given the stream
   // tensor maps for the fast kernel (encoded for one tile shape)
   CUtensorMap tm_halo[2], tm_own[2], tm_c[4];  // tm_c: L, O1, O2, row bases
   int fast_slots = 0;      // fast-sweep CTAs resident on the device at once

@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(128, 8) lb_tc_kernel(const float *__restrict__
 // tanh per tile).  Sixteen lines per warp, because neighbours in the table
 // are neighbours in x on four of the six faces: one gather instruction brings
 // two 128-byte runs (with four lines eight 32-byte ones).  [line][cell] in
-// shared memory and weight fragments shared by two tiles issue 60 wavefronts
+// shared memory and weight fragments shared by two tiles issue 70 wavefronts
 // per tile where [cell][line] and a tile at a time issued 130 (82 % of the
 // pipe); that costs registers, so four CTAs per SM instead of eight.
 constexpr int kLine = kCorrected;               // corrected cells per line

@@ -92,6 +92,17 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map,
       : "memory");
 }
 
+// Programmatic dependent launch.  wait: until every grid this one was launched
+// after has completed and its writes are visible (returns at once when the
+// launch has no programmatic dependency).  launch: the next grid of the stream
+// may start once every CTA of this one has called it or left.
+__device__ __forceinline__ void grid_dep_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dep_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(
                    reinterpret_cast<uint64_t>(map))

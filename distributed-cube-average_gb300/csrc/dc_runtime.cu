@@ -81,7 +81,12 @@ T *direct_view(T *p, int dev) {
   }
 }
 
-Sim *impl(dc_gb300_sim *h) { return h ? h->impl : nullptr; }
+// The simulation of an API call.  Any call but a propagate ends the run of
+// boxes that may be computed beside one another.
+Sim *impl(dc_gb300_sim *h) {
+  if (h && h->impl) h->impl->boxes.clear();
+  return h ? h->impl : nullptr;
+}
 
 // Pair buffer that holds the field whose p component is `p` and q component
 // `q` (q == p + 1), or -1.
@@ -516,6 +521,7 @@ extern "C" long dc_gb300_device_pitch(const dc_gb300_sim *h) {
 }
 
 extern "C" void *dc_gb300_stream(dc_gb300_sim *h) {
+  if (Sim *s = impl(h)) s->stream_shared = true;
   return h && h->impl ? static_cast<void *>(h->impl->stream) : nullptr;
 }
 
@@ -1376,10 +1382,26 @@ extern "C" int dc_gb300_synchronize(dc_gb300_sim *h) {
   return check_err_word(s);
 }
 
-extern "C" int dc_gb300_propagate_box(dc_gb300_sim *h, const size_t start[3],
-                                      const size_t end[3]) {
-  Sim *s = impl(h);
-  if (!s || !start || !end) return fail(DC_GB300_ERR_ARG, "null argument");
+namespace {
+
+// Whether the box [b0, b1) may be computed beside the passes still in flight:
+// they are boxes of the same step (same roles, no other call in between) and
+// share no point with it, so none reads what another writes.  Notes the box.
+bool runs_beside(Sim *s, const long long b0[3], const long long b1[3]) {
+  const dc_device_data &a = s->handle->abi;
+  if (a.pp != s->box_pp || a.pc != s->box_pc) s->boxes.clear();
+  s->box_pp = a.pp;
+  s->box_pc = a.pc;
+  bool apart = !s->boxes.empty() && !s->stream_shared;
+  for (const auto &o : s->boxes)
+    apart = apart && (b0[0] >= o[3] || o[0] >= b1[0] || b0[1] >= o[4] || o[1] >= b1[1] ||
+                      b0[2] >= o[5] || o[2] >= b1[2]);
+  if (!apart) s->boxes.clear();  // this pass waits for all before it
+  s->boxes.push_back({b0[0], b0[1], b0[2], b1[0], b1[1], b1[2]});
+  return apart;
+}
+
+int propagate_box(Sim *s, const size_t start[3], const size_t end[3]) {
   const long long lim[3] = {s->sx, s->sy, s->sz};
   long long b0[3], b1[3];
   for (int d = 0; d < 3; ++d) {
@@ -1393,13 +1415,27 @@ extern "C" int dc_gb300_propagate_box(dc_gb300_sim *h, const size_t start[3],
   if (!roles(s, &cur, &prev))
     return fail(DC_GB300_ERR_STATE, "field pointers do not belong to this simulation");
   DCG_TRY(cudaSetDevice(s->device));
+  StepParams p;
   if (s->kernel == DC_GB300_KERNEL_FAST) {
+    // (a 16-bit copy of the medium is refreshed first)
+    if (s->coef16 && s->coef16_stale) s->boxes.clear();
     const int rc = refresh_narrow(s);
     if (rc != DC_GB300_OK) return rc;
+    p = make_params(s, b0, b1, s->dx, s->dy, s->dz, s->dt);
+    p.beside = runs_beside(s, b0, b1) ? 1 : 0;
+  } else {
+    p = make_params(s, b0, b1, s->dx, s->dy, s->dz, s->dt);
   }
-  StepParams p = make_params(s, b0, b1, s->dx, s->dy, s->dz, s->dt);
   DCG_TRY(launch_pass(s, p));
   return DC_GB300_OK;
+}
+
+}  // namespace
+
+extern "C" int dc_gb300_propagate_box(dc_gb300_sim *h, const size_t start[3],
+                                      const size_t end[3]) {
+  if (!h || !h->impl || !start || !end) return fail(DC_GB300_ERR_ARG, "null argument");
+  return propagate_box(h->impl, start, end);
 }
 
 // ===========================================================================
@@ -1504,7 +1540,7 @@ extern "C" void dc_propagate(const size_t start_coords[3], const size_t end_coor
                              dc_device_data *data, const float dx, const float dy,
                              const float dz, const float dt) {
   dc_gb300_sim *h = dc_gb300_from_device_data(data);
-  Sim *s = impl(h);
+  Sim *s = h ? h->impl : nullptr;
   if (!s || !sizes || static_cast<long long>(sizes[0]) != s->sx ||
       static_cast<long long>(sizes[1]) != s->sy || static_cast<long long>(sizes[2]) != s->sz) {
     set_error("sizes differ from the ones given to dc_device_data_init");
@@ -1515,7 +1551,11 @@ extern "C" void dc_propagate(const size_t start_coords[3], const size_t end_coor
   s->dy = dy;
   s->dz = dz;
   s->dt = dt;
-  if (dc_gb300_propagate_box(h, start_coords, end_coords) != DC_GB300_OK)
+  if (!start_coords || !end_coords) {
+    set_error("null argument");
+    abi_die("dc_propagate");
+  }
+  if (propagate_box(s, start_coords, end_coords) != DC_GB300_OK)
     abi_die("dc_propagate");
 }
 

@@ -456,6 +456,11 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
     if (Lay::VB_PLANE) prefetch_tensormap(tm_vb);
   }
   __syncthreads();
+  // Everything above ran while the previous grid of the stream was finishing;
+  // its fields are read and overwritten from here on.  Only then may the next
+  // one be brought in: one grid waits at a time.
+  if (!prm.beside) grid_dep_wait();
+  grid_dep_launch();
 
   // Producer: one elected thread fills stage s with the group of iterations
   // j .. j + GROUP - 1, one copy per array (planes past the array read
@@ -802,6 +807,7 @@ __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
   extern __shared__ __align__(1024) unsigned char smem[];
   if (smem_u32(smem) & 127u) {
     if (threadIdx.x == 0) atomicOr(prm.err, kErrAlign);
+    grid_dep_wait();
     return;
   }
   const int x0 = prm.tile_x0 + static_cast<int>(blockIdx.x) * TX;
@@ -810,6 +816,9 @@ __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
   const int ze = min(zb + prm.zchunk, prm.z1);
   sweep_column<TX, TY, CF, SPONGE, ISO>(&tm_cur, &tm_prev, &tm_l, &tm_o1, &tm_o2, &tm_vb, prm,
                                         prm, x0, y0, zb, ze, smem);
+  // beside another pass: done only when that one is, so that whoever waits for
+  // this grid waits for all boxes of the step
+  if (prm.beside) grid_dep_wait();
 }
 
 // One step of a batch of shots: persistent CTAs stride over the work items
@@ -855,10 +864,22 @@ cudaError_t launch_fast_t(Sim *sim, const StepParams &prm, int cur_buf, int prev
   const int nx = prm.x1 - prm.tile_x0, ny = prm.y1 - prm.tile_y0;
   const int nz = prm.z1 - prm.z0;
   dim3 grid((nx + kTX - 1) / kTX, (ny + kTY - 1) / kTY, (nz + prm.zchunk - 1) / prm.zchunk);
-  fast_kernel<kTX, kTY, kCF, SPONGE, ISO><<<grid, Lay::NT, Lay::SMEM_BYTES, sim->stream>>>(
-      sim->tm_halo[cur_buf], sim->tm_own[prev_buf], sim->tm_c[0], sim->tm_c[1], sim->tm_c[2],
-      sim->tm_c[3], prm);  // tm_c: L, O1, O2, row bases
-  return cudaGetLastError();
+  // Programmatic dependent launch: the grid is set up (and its CTAs' tensor
+  // maps and barriers are made ready) while the previous one finishes.
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(Lay::NT);
+  cfg.dynamicSmemBytes = Lay::SMEM_BYTES;
+  cfg.stream = sim->stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  // tm_c: L, O1, O2, row bases
+  return cudaLaunchKernelEx(&cfg, fast_kernel<kTX, kTY, kCF, SPONGE, ISO>, sim->tm_halo[cur_buf],
+                            sim->tm_own[prev_buf], sim->tm_c[0], sim->tm_c[1], sim->tm_c[2],
+                            sim->tm_c[3], prm);
 }
 
 cudaError_t launch_one(Sim *sim, const StepParams &prm, int cur, int prev) {

@@ -96,3 +96,39 @@ def test_short_chunks_change_no_bit(dc, monkeypatch, sizes):
     for f, tr in outs[1:]:
         assert all(np.array_equal(f[k], outs[0][0][k]) for k in f)
         assert np.array_equal(tr, outs[0][1])
+
+
+@pytest.mark.parametrize("medium", ["PRECOMP", "PRECOMP_F16", "VPZ_VSV"])
+def test_boxes_beside_one_another(dc, medium):
+    """Disjoint boxes of a step run beside one another, anything else waits:
+    the same calls with a synchronisation after each give the same bits.  The
+    overlapping and repeated boxes read what the calls before them wrote."""
+    sizes = (88, 72, 64)
+    form = getattr(dc, "MEDIUM_" + medium)
+    coef, fields = inputs(sizes, 9)
+    sx, sy, sz = sizes
+    step = [((4, 4, 4), (8, sy - 4, sz - 4)), ((sx - 8, 4, 4), (sx - 4, sy - 4, sz - 4)),
+            ((8, 4, 4), (sx - 8, 8, sz - 4)), ((8, sy - 8, 4), (sx - 8, sy - 4, sz - 4)),
+            ((8, 8, 4), (sx - 8, sy - 8, 8)), ((8, 8, sz - 8), (sx - 8, sy - 8, sz - 4)),
+            ((9, 9, 9), (9, 40, 40)), ((8, 8, 8), (sx - 8, sy - 8, sz - 8))]
+    odd = [((7, 9, 10), (40, 41, 30)), ((39, 9, 10), (50, 41, 30)), ((60, 9, 10), (61, 10, 11)),
+           ((60, 9, 10), (61, 10, 11)), ((7, 9, 10), (40, 41, 30))]
+    outs = []
+    for wait in (True, False, False):
+        with dc.Simulation(sizes, (12.5,) * 3, 1e-3, medium=form, device=0) as sim:
+            if medium == "VPZ_VSV":
+                sim.set_vpz_vsv(np.sqrt(coef[6]), 0.4 * np.sqrt(coef[7]))
+            else:
+                sim.set_precomp(coef)
+            sim.set_fields(*fields)
+            for _ in range(10):
+                for boxes in (step, odd):
+                    for b0, b1 in boxes:
+                        sim.propagate_box(b0, b1)
+                        if wait:
+                            sim.synchronize()
+                    dc.device_swap_arrays(sim.device_data)
+            sim.synchronize()
+            outs.append(sim.get_fields())
+    for o in outs[1:]:
+        assert all(np.array_equal(o[k], outs[0][k]) for k in o)
