@@ -200,6 +200,25 @@ struct Sim {
   int graph_pc[2] = {-1, -1};
 };
 
+// Launches `kernel` with a programmatic dependency on the previous grid of the
+// stream: it is set up while that one finishes.  The kernel must call
+// grid_dep_wait() before it touches what that grid reads or writes.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
+                             cudaStream_t st, A &&...args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // The kernels of the fast sweep for one coefficient form and tile height:
 // tti_fast_inst.cu is compiled once per pair and specialises fast_ops.
 struct FastOps {

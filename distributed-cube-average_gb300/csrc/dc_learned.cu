@@ -43,6 +43,7 @@
 #include <vector>
 
 #include "dc_internal.h"
+#include "dc_ptx.cuh"
 
 namespace dcg {
 namespace {
@@ -192,7 +193,7 @@ __device__ __forceinline__ void outer128(const float *d, const float *x, float g
     for (int j = 0; j < 2; ++j) g[o][j] += s[o][j];
 }
 
-__global__ void __launch_bounds__(kTT) mlp_grad_kernel(const float *__restrict__ wc,
+__global__ void __launch_bounds__(kTT) mlp_grad_kernel(const float *wc,
                                                        const float *__restrict__ xs,
                                                        const float *__restrict__ ts, long long n,
                                                        long long count, unsigned long long seed,
@@ -200,17 +201,20 @@ __global__ void __launch_bounds__(kTT) mlp_grad_kernel(const float *__restrict__
   extern __shared__ __align__(16) unsigned char grad_smem[];
   GradSmem &sm = *reinterpret_cast<GradSmem *>(grad_smem);
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  for (int i = t; i < kHid * kIn; i += kTT) {
-    // (transposed: the reads are scattered over the 4 KB, the stores are not)
-    const int k = i / kHid, o = i % kHid;
-    sm.w1t[i] = wc[OFF_W1 + o * kIn + k];
-    sm.w2t[i] = wc[OFF_W2 + o * kHid + k];
-    sm.w2[i] = wc[OFF_W2 + i];
-  }
-  for (int i = t; i < kDepths * kHid; i += kTT) sm.b1[i] = wc[OFF_B1 + i];
-  if (t < kOut * kHid) sm.w3[t] = wc[OFF_W3 + t];
-  if (t < kHid) sm.b2[t] = wc[OFF_B2 + t];
-  if (t < kOut) sm.b3[t] = wc[OFF_B3 + t];
+  auto stage = [&] {
+    for (int i = t; i < kHid * kIn; i += kTT) {
+      // (transposed: the reads are scattered over the 4 KB, the stores are not)
+      const int k = i / kHid, o = i % kHid;
+      sm.w1t[i] = wc[OFF_W1 + o * kIn + k];
+      sm.w2t[i] = wc[OFF_W2 + o * kHid + k];
+      sm.w2[i] = wc[OFF_W2 + i];
+    }
+    for (int i = t; i < kDepths * kHid; i += kTT) sm.b1[i] = wc[OFF_B1 + i];
+    if (t < kOut * kHid) sm.w3[t] = wc[OFF_W3 + t];
+    if (t < kHid) sm.b2[t] = wc[OFF_B2 + t];
+    if (t < kOut) sm.b3[t] = wc[OFF_B3 + t];
+  };
+  bool staged = false;
   // gradients of this thread: units go, go + 1 x inputs gk, gk + 16 of W1
   // (warps 0-7) or W2 (8-15); unit `lane` at depth w of b1; W3 (warps 0, 1),
   // b2 (2) and b3 (3)
@@ -241,6 +245,12 @@ __global__ void __launch_bounds__(kTT) mlp_grad_kernel(const float *__restrict__
     for (int q = 0; q < 8; q += 4)
       *reinterpret_cast<float4 *>(sm.xh + lane * kRow + 8 * w + q) =
           make_float4(x[q], x[q + 1], x[q + 2], x[q + 3]);
+    if (!staged) {  // the first rows come in while Adam updates the weights
+      grid_dep_wait();
+      grid_dep_launch();
+      stage();
+      staged = true;
+    }
     __syncthreads();
     if (t < kTB) {
       float ss = 0.f;
@@ -393,10 +403,10 @@ __global__ void __launch_bounds__(kTT) mlp_grad_kernel(const float *__restrict__
 // gradient kernel instead, the step took 20 us longer).
 constexpr int kAdamT = 64;
 __global__ void __launch_bounds__(kAdamT)
-    mlp_adam_kernel(float *__restrict__ master, float *__restrict__ wc, float *__restrict__ m1,
-                    float *__restrict__ m2, float *__restrict__ grad,
-                    const double *__restrict__ acc, double *__restrict__ next_acc, float lr,
-                    float b1, float b2, float eps, int step, float *loss_hist, int hist_index) {
+    mlp_adam_kernel(float *master, float *wc, float *m1, float *m2, float *grad,
+                    const double *acc, double *next_acc, float lr, float b1, float b2, float eps, int step, float *loss_hist, int hist_index) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int p = blockIdx.x * kAdamT + threadIdx.x;
   const double w = acc[1];
   if (p < kParams) {
@@ -795,6 +805,8 @@ __global__ void __launch_bounds__(128, 8) lb_tc_kernel(const float *__restrict__
                                                        long long n, float2 *out) {
   __shared__ NetSmem sm;
   stage_net(wc, sm);
+  grid_dep_wait();  // the fields of the launch before
+  grid_dep_launch();
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -913,6 +925,8 @@ __global__ void __launch_bounds__(128, kLineCtas)
     }
   };
   long long base = warp * kLineWarp;
+  grid_dep_wait();  // the weights are staged while the stencil finishes
+  grid_dep_launch();
   if (base >= nlines) return;  // (no CTA barrier below)
   LinePtr now = pointers(entry(base)), next = pointers(entry(base + stride));
   int4 after = entry(base + 2 * stride);
@@ -966,7 +980,9 @@ __global__ void __launch_bounds__(128, kLineCtas)
 }
 
 template <class Entries>
-__global__ void lb_add_edge_kernel(Entries src, long long n, const float2 *__restrict__ corr) {
+__global__ void lb_add_edge_kernel(Entries src, long long n, const float2 *corr) {
+  grid_dep_wait();
+  grid_dep_launch();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float2 *p = src.at(src.table[i]).nw;
@@ -1167,17 +1183,16 @@ template <class Entries>
 cudaError_t launch_entries(cudaStream_t st, const float *wc, int layer, Entries lines,
                            long long nl, Entries edge, long long ne, float2 *corr) {
   if (nl > 0) {
-    lb_line_kernel<Entries><<<line_grid(nl), 128, 0, st>>>(wc, lines, nl, layer);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_dependent(lb_line_kernel<Entries>, dim3(line_grid(nl)), 128, 0, st,
+                                           wc, lines, nl, layer);
     if (e != cudaSuccess) return e;
   }
   if (ne <= 0) return cudaSuccess;
-  lb_tc_kernel<EdgeSrc<Entries>><<<grid_for(ne, 64), 128, 0, st>>>(wc, EdgeSrc<Entries>{edge}, ne,
-                                                                   corr);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_dependent(lb_tc_kernel<EdgeSrc<Entries>>, dim3(grid_for(ne, 64)),
+                                         128, 0, st, wc, EdgeSrc<Entries>{edge}, ne, corr);
   if (e != cudaSuccess) return e;
-  lb_add_edge_kernel<Entries><<<grid_for(ne, 256), 256, 0, st>>>(edge, ne, corr);
-  return cudaGetLastError();
+  return launch_dependent(lb_add_edge_kernel<Entries>, dim3(grid_for(ne, 256)), 256, 0, st, edge,
+                          ne, corr);
 }
 
 }  // namespace
@@ -1400,14 +1415,15 @@ extern "C" int dc_gb300_mlp_train(dc_gb300_mlp *m, const float *samples, const f
   const int blocks = dcg::grid_for(batch, dcg::kTB);
   for (int s = 0; s < steps && e == cudaSuccess; ++s) {
     double *acc = m->acc + 2 * (s & 1), *next = m->acc + 2 * (1 - (s & 1));
-    dcg::mlp_grad_kernel<<<blocks, dcg::kTT, sizeof(dcg::GradSmem), m->stream>>>(
-        m->wc, samples, targets, n, batch, seed + 0x9E3779B97F4A7C15ull * (m->adam_step + 1), 1,
-        m->grad, acc);
+    e = dcg::launch_dependent(dcg::mlp_grad_kernel, dim3(blocks), dcg::kTT, sizeof(dcg::GradSmem),
+                              m->stream, m->wc, samples, targets, n, batch,
+                              seed + 0x9E3779B97F4A7C15ull * (m->adam_step + 1), 1, m->grad, acc);
+    if (e != cudaSuccess) break;
     ++m->adam_step;
-    dcg::mlp_adam_kernel<<<(dcg::kParams + dcg::kAdamT - 1) / dcg::kAdamT, dcg::kAdamT, 0,
-                           m->stream>>>(m->master, m->wc, m->m1, m->m2, m->grad, acc, next, lr,
-                                        0.9f, 0.999f, 1e-8f, m->adam_step, d_hist, s);
-    e = cudaGetLastError();
+    e = dcg::launch_dependent(dcg::mlp_adam_kernel,
+                              dim3((dcg::kParams + dcg::kAdamT - 1) / dcg::kAdamT), dcg::kAdamT, 0,
+                              m->stream, m->master, m->wc, m->m1, m->m2, m->grad, acc, next, lr,
+                              0.9f, 0.999f, 1e-8f, m->adam_step, d_hist, s);
   }
   if (e == cudaSuccess && d_hist)
     e = cudaMemcpyAsync(loss_hist, d_hist, sizeof(float) * steps, cudaMemcpyDeviceToHost,

@@ -864,22 +864,10 @@ cudaError_t launch_fast_t(Sim *sim, const StepParams &prm, int cur_buf, int prev
   const int nx = prm.x1 - prm.tile_x0, ny = prm.y1 - prm.tile_y0;
   const int nz = prm.z1 - prm.z0;
   dim3 grid((nx + kTX - 1) / kTX, (ny + kTY - 1) / kTY, (nz + prm.zchunk - 1) / prm.zchunk);
-  // Programmatic dependent launch: the grid is set up (and its CTAs' tensor
-  // maps and barriers are made ready) while the previous one finishes.
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(Lay::NT);
-  cfg.dynamicSmemBytes = Lay::SMEM_BYTES;
-  cfg.stream = sim->stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
   // tm_c: L, O1, O2, row bases
-  return cudaLaunchKernelEx(&cfg, fast_kernel<kTX, kTY, kCF, SPONGE, ISO>, sim->tm_halo[cur_buf],
-                            sim->tm_own[prev_buf], sim->tm_c[0], sim->tm_c[1], sim->tm_c[2],
-                            sim->tm_c[3], prm);
+  return launch_dependent(fast_kernel<kTX, kTY, kCF, SPONGE, ISO>, grid, Lay::NT, Lay::SMEM_BYTES,
+                          sim->stream, sim->tm_halo[cur_buf], sim->tm_own[prev_buf],
+                          sim->tm_c[0], sim->tm_c[1], sim->tm_c[2], sim->tm_c[3], prm);
 }
 
 cudaError_t launch_one(Sim *sim, const StepParams &prm, int cur, int prev) {
@@ -940,19 +928,13 @@ int occ_batch(bool iso, bool sponge) {
 
 cudaError_t launch_batch_one(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
                              int blocks) {
-  bool done = false;
+  auto go = [&](auto kernel) {
+    return launch_dependent(kernel, dim3(blocks), Lay::NT, Lay::SMEM_BYTES, st, bl);
+  };
   if constexpr (kNoSponge)
-    if (iso && !sponge) {
-      batch_kernel<kTX, kTY, kCF, false, true><<<blocks, Lay::NT, Lay::SMEM_BYTES, st>>>(bl);
-      done = true;
-    }
-  if (!done) {
-    if (iso)
-      batch_kernel<kTX, kTY, kCF, true, true><<<blocks, Lay::NT, Lay::SMEM_BYTES, st>>>(bl);
-    else
-      batch_kernel<kTX, kTY, kCF, true, false><<<blocks, Lay::NT, Lay::SMEM_BYTES, st>>>(bl);
-  }
-  return cudaGetLastError();
+    if (iso && !sponge) return go(batch_kernel<kTX, kTY, kCF, false, true>);
+  return iso ? go(batch_kernel<kTX, kTY, kCF, true, true>)
+             : go(batch_kernel<kTX, kTY, kCF, true, false>);
 }
 
 }  // namespace
