@@ -132,3 +132,40 @@ def test_boxes_beside_one_another(dc, medium):
             outs.append(sim.get_fields())
     for o in outs[1:]:
         assert all(np.array_equal(o[k], outs[0][k]) for k in o)
+
+
+@pytest.mark.parametrize("medium", [0, 1])
+def test_exact_kernel_edges_and_alignment(dc, medium):
+    """Two columns per lane give the bits of one column per lane, which takes
+    buffers that are not 16-byte aligned: the same boxes through both, over
+    ragged sizes."""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    for sizes in ((9, 9, 9), (10, 12, 26), (43, 17, 11), (44, 9, 25)):
+        sx, sy, sz = sizes
+        pitch = (sx + 3) // 4 * 4
+        count = pitch * sy * sz
+        g = torch.Generator("cuda").manual_seed(sum(sizes))
+        per = 10 if medium == 0 else 2
+        med = torch.rand(count * per, generator=g, device="cuda") * 0.5
+        first = [torch.randn(count * 2 + 2, generator=g, device="cuda") for _ in range(2)]
+        outs = []
+        for shift in (0, 2):  # floats: 16-byte aligned, and 8 bytes off
+            bufs = []
+            for f in first:
+                b = torch.zeros(count * 2 + 8, device="cuda")
+                b[shift:shift + count * 2] = f[:count * 2]
+                bufs.append(b)
+            cfg = dc.Config(sx, sy, sz, 2.0, 1.5, 1.25, 0.5, dc.KERNEL_EXACT, medium, 0)
+            pairs = (C.c_void_p * 2)(*[b.data_ptr() + 4 * shift for b in bufs])
+            steps = 3
+            energy = np.zeros(steps)
+            torch.cuda.synchronize()
+            dc.check(dc.lib().dc_gb300_exact_steps_noalloc(
+                C.byref(cfg), pairs, med.data_ptr(), steps,
+                energy.ctypes.data_as(C.POINTER(C.c_double)), None))
+            outs.append([b[shift:shift + count * 2].cpu().numpy() for b in bufs] + [energy])
+        a, b = outs
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+        assert np.allclose(a[2], b[2], rtol=1e-6, atol=0)
