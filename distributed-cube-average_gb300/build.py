@@ -39,16 +39,17 @@ def nvcc() -> str:
 
 
 # the fast sweep's kernels: one translation unit per coefficient form and
-# tile height (each takes tens of seconds; in one file they would be serial)
+# tile shape (each takes tens of seconds; in one file they would be serial)
 FAST = CSRC / "tti_fast_inst.cu"
-FAST_UNITS = [(form, ty) for form in ("CF_F32", "CF_F16", "CF_BF16", "CF_VV") for ty in (8, 16)]
+FAST_UNITS = [(form, tx, ty) for tx, ty in ((32, 8), (32, 16), (16, 16))
+              for form in ("CF_F32", "CF_F16", "CF_BF16", "CF_VV")]
 
 
 def sources() -> list[tuple[Path, list[str], str]]:
     """(source, defines, object name) of every translation unit, the slow
     ones first."""
-    units = [(FAST, [f"-DDC_FORM={form}", f"-DDC_TY={ty}"], f"{FAST.stem}_{form}_{ty}.o")
-             for form, ty in FAST_UNITS]
+    units = [(FAST, [f"-DDC_FORM={form}", f"-DDC_TX={tx}", f"-DDC_TY={ty}"],
+              f"{FAST.stem}_{form}_{tx}x{ty}.o") for form, tx, ty in FAST_UNITS]
     rest = sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cpp")))
     return units + [(s, [], s.name + ".o") for s in rest if s != FAST]
 

@@ -237,13 +237,13 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
   std::string err;
   CUtensorMap tm_c[4];
   if (!fast_encode_medium_maps(b->coef_form, b->coef, b->coef16, nullptr, b->vbase, b->mx,
-                               b->my, b->mz, b->mpitch, b->mcount, ty, tm_c, &err))
+                               b->my, b->mz, b->mpitch, b->mcount, kFastTX, ty, tm_c, &err))
     return fail(DC_GB300_ERR_CUDA, err);
   std::vector<CUtensorMap> maps(static_cast<size_t>(n) * 4);
   for (int i = 0; i < n; ++i) {
     const BShot &s = b->shots[i];
     for (int buf = 0; buf < 2; ++buf)
-      if (!fast_encode_pair_maps(s.pq[buf], s.cfg.sx, s.cfg.sy, s.cfg.sz, s.pitch, ty,
+      if (!fast_encode_pair_maps(s.pq[buf], s.cfg.sx, s.cfg.sy, s.cfg.sz, s.pitch, kFastTX, ty,
                                  &maps[4 * i + buf], &maps[4 * i + 2 + buf], &err))
         return fail(DC_GB300_ERR_CUDA, err);
   }

@@ -131,6 +131,12 @@ struct BatchLaunch {
   StepParams shot[kMaxBatchShots];
 };
 
+// Tensor maps of a box for one tile shape: the pair buffers with halo and
+// without, and the medium's groups (L, O1, O2, row bases).
+struct FastMaps {
+  CUtensorMap halo[2], own[2], c[4];
+};
+
 struct Sim {
   dc_gb300_sim *handle = nullptr;
   int device = 0;
@@ -179,8 +185,8 @@ struct Sim {
   std::vector<std::array<long long, 6>> boxes;
   const float *box_pp = nullptr, *box_pc = nullptr;
   bool stream_shared = false;  // the caller has been given the stream
-  // tensor maps for the fast kernel (encoded for one tile shape)
-  CUtensorMap tm_halo[2], tm_own[2], tm_c[4];  // tm_c: L, O1, O2, row bases
+  // tensor maps for the fast kernel: its tiles, and the strip's
+  FastMaps maps, strip_maps;
   int fast_slots = 0;      // fast-sweep CTAs resident on the device at once
   int maps_tx = 0, maps_ty = 0;
   // learned absorbing layer, applied after every stencil pass of a run
@@ -219,18 +225,35 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// The kernels of the fast sweep for one coefficient form and tile height:
-// tti_fast_inst.cu is compiled once per pair and specialises fast_ops.
+// The kernels of the fast sweep for one coefficient form and tile shape:
+// tti_fast_inst.cu is compiled once per combination and specialises fast_ops.
 struct FastOps {
   cudaError_t (*attrs)();  // shared-memory attributes
   int (*occupancy)();      // CTAs per SM
-  cudaError_t (*launch)(Sim *sim, const StepParams &prm, int cur_buf, int prev_buf);
+  cudaError_t (*launch)(const Sim *sim, const FastMaps &maps, const StepParams &prm, int cur_buf,
+                        int prev_buf);
+  // (32-column tiles only)
   cudaError_t (*batch_attrs)();
   int (*batch_occupancy)(bool iso, bool sponge);
   cudaError_t (*launch_batch)(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
                               int blocks);
 };
-constexpr int kFastTX = 32;  // tile width: half a warp of two-point lanes
+constexpr int kFastTX = 32;                // tile width: half a warp of two-point lanes
+constexpr int kStripTX = 16, kStripTY = 16;  // tiles of a narrow last column
+template <int FORM, int TX, int TY>
+const FastOps &fast_ops();
+#define DCG_DECL_OPS(f)                  \
+  template <>                            \
+  const FastOps &fast_ops<f, 32, 8>();   \
+  template <>                            \
+  const FastOps &fast_ops<f, 32, 16>();  \
+  template <>                            \
+  const FastOps &fast_ops<f, 16, 16>()
+DCG_DECL_OPS(CF_F32);
+DCG_DECL_OPS(CF_VV);
+DCG_DECL_OPS(CF_F16);
+DCG_DECL_OPS(CF_BF16);
+#undef DCG_DECL_OPS
 constexpr int kGroup = 3;    // planes of a TMA copy, and between two CTA barriers
 template <int FORM, int TY>
 const FastOps &fast_ops();
@@ -252,23 +275,25 @@ struct FastShape {
 // Tile shape and z-chunk of a fast pass over an nx x ny x nz box.
 FastShape fast_shape(const Sim *sim, long long nx, long long ny, long long nz);
 bool fast_encode_maps(Sim *sim, std::string *err);
+// Kernel launches of a fast pass over nx columns (from tile_x0) and ny rows.
+int fast_launches(const Sim *sim, long long nx, long long ny);
 // Tile rows (TY) of the fast kernel for coefficient form `form`: 8 unless
 // DC_GB300_FAST_TY selects 16.
 int fast_default_ty(int form);
 // Whether tile rows `ty` are compiled for coefficient form `form` (8 and 16).
 bool fast_tile_rows_valid(int ty, int form);
-// Tensor maps of one (p, q) pair buffer for tiles of 32 x ty: the halo box
+// Tensor maps of one (p, q) pair buffer for tiles of tx x ty: the halo box
 // (read as the current field) and the own tile (previous field).
 bool fast_encode_pair_maps(const float2 *buf, long long sx, long long sy, long long sz,
-                           long long pitch, int ty, CUtensorMap *halo, CUtensorMap *own,
+                           long long pitch, int tx, int ty, CUtensorMap *halo, CUtensorMap *own,
                            std::string *err);
 // Tensor maps of the three coefficient groups of a medium in form `form`.
 // out[0..2] = the groups L, O1, O2; out[3] = the FP16 form's row bases
 // (vbase, [sz][sy] float4; a copy of out[2] for the other forms).
 bool fast_encode_medium_maps(int form, const float *coef, const void *coef16, const float *vv,
                              const float4 *vbase, long long sx, long long sy, long long sz,
-                             long long pitch, long long count, int ty, CUtensorMap out[4],
-                             std::string *err);
+                             long long pitch, long long count, int tx, int ty,
+                             CUtensorMap out[4], std::string *err);
 // Batched fast kernel (always with the sponge).  `blocks` = persistent CTAs.
 cudaError_t batch_prepare(int ty, int form);  // shared-memory attributes
 // `sponge` false: every shot's sponge profile is 1 (the no-sponge sweep)

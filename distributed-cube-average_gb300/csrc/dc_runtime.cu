@@ -260,8 +260,11 @@ StepParams make_params(Sim *s, const long long b0[3], const long long b1[3],
 }
 
 cudaError_t launch_pass(Sim *s, const StepParams &p) {
-  ++s->launches;
-  if (s->kernel == DC_GB300_KERNEL_EXACT) return launch_exact(s, p);
+  if (s->kernel == DC_GB300_KERNEL_EXACT) {
+    ++s->launches;
+    return launch_exact(s, p);
+  }
+  s->launches += fast_launches(s, p.x1 - p.tile_x0, p.y1 - p.tile_y0);
   int cur = -1, prev = -1;
   roles(s, &cur, &prev);  // checked by the callers
   return launch_fast(s, p, cur, prev);
@@ -275,8 +278,10 @@ void swap_roles(dc_device_data *a) {
 // Kernel launches of one step: the stencil pass, then with a learned layer
 // the face-line pass and the edge cells' network and add.
 long long launches_per_step(const Sim *s) {
-  if (s->lb_cells <= 0) return 1;
-  return 1 + (s->lb_lines > 0 ? 1 : 0) + (s->lb_edge > 0 ? 2 : 0);
+  const long long stencil =
+      s->kernel == DC_GB300_KERNEL_FAST ? fast_launches(s, s->sx - 8, s->sy - 8) : 1;
+  if (s->lb_cells <= 0) return stencil;
+  return stencil + (s->lb_lines > 0 ? 1 : 0) + (s->lb_edge > 0 ? 2 : 0);
 }
 
 // Queues one full time step (j-th of a run): fused source for the next
@@ -319,7 +324,7 @@ cudaError_t queue_step(Sim *s, int j) {
       e = launch_lb_step(s->stream, s->lb_params, s->d_lb_cells, s->lb_cells, s->pq[prev],
                          s->pq[cur], s->pitch, s->plane, s->d_lb_corr, s->lb_rec);
     } else {
-      s->launches += launches_per_step(s) - 1;
+      s->launches += (s->lb_lines > 0 ? 1 : 0) + (s->lb_edge > 0 ? 2 : 0);
       e = launch_lb_fused(s->stream, s->lb_params, s->lb_layer, s->d_lb_lines, s->lb_lines,
                           s->d_lb_edge, s->lb_edge, s->pq[prev], s->pq[cur], s->d_lb_corr);
     }

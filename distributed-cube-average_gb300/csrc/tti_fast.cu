@@ -11,14 +11,26 @@ namespace {
 
 constexpr int kTX = kFastTX;
 
-// The kernels of a coefficient form and tile height (8 or 16 rows).
+// The kernels of a coefficient form and tile height (8 or 16 rows of 32), and
+// of its strips.
+template <int FORM>
+const FastOps &ops_of(int ty) {
+  return ty == 16 ? fast_ops<FORM, kTX, 16>() : fast_ops<FORM, kTX, 8>();
+}
 const FastOps &ops_for(int form, int ty) {
-  const bool tall = ty == 16;
   switch (form) {
-    case CF_VV: return tall ? fast_ops<CF_VV, 16>() : fast_ops<CF_VV, 8>();
-    case CF_F16: return tall ? fast_ops<CF_F16, 16>() : fast_ops<CF_F16, 8>();
-    case CF_BF16: return tall ? fast_ops<CF_BF16, 16>() : fast_ops<CF_BF16, 8>();
-    default: return tall ? fast_ops<CF_F32, 16>() : fast_ops<CF_F32, 8>();
+    case CF_VV: return ops_of<CF_VV>(ty);
+    case CF_F16: return ops_of<CF_F16>(ty);
+    case CF_BF16: return ops_of<CF_BF16>(ty);
+    default: return ops_of<CF_F32>(ty);
+  }
+}
+const FastOps &strip_ops(int form) {
+  switch (form) {
+    case CF_VV: return fast_ops<CF_VV, kStripTX, kStripTY>();
+    case CF_F16: return fast_ops<CF_F16, kStripTX, kStripTY>();
+    case CF_BF16: return fast_ops<CF_BF16, kStripTX, kStripTY>();
+    default: return fast_ops<CF_F32, kStripTX, kStripTY>();
   }
 }
 
@@ -30,6 +42,33 @@ int chosen_ty(int) {
   const char *e = std::getenv("DC_GB300_FAST_TY");
   const int v = e ? std::atoi(e) : 0;
   return v == 16 ? 16 : 8;
+}
+
+long long div_up(long long a, long long b) { return (a + b - 1) / b; }
+
+// CTAs of the fast sweep resident on the device at once.
+long long slots_of(const Sim *sim) { return sim->fast_slots > 0 ? sim->fast_slots : 2 * 152; }
+
+// Whether the last nx % 32 columns of a pass go to a launch of 16 x 16 tiles
+// beside the one of 32 x 8 tiles: when they fit 16 columns, where a 32-column
+// tile would compute more padding than points.  Per step without / with: 240 x
+// 222 x 251 BF16 (8 of 232 columns left over) 114 / 110 us, 408^3 vpz/vsv (16 of
+// 400) 541 / 525 us.  The FP32 ten-coefficient form waits for HBM, not for the
+// padding's arithmetic (307 x 291 x 299: 255 / 262 us), and a box that does not
+// give every SM a CTA takes as long as one CTA, however many there are: neither
+// has a second launch.  A single narrow column (the x faces of the seven-box
+// loop) is one launch of 16 x 16 tiles in every form.
+bool has_strip(const Sim *sim, long long nx, long long ny) {
+  const long long rest = nx % kTX;
+  if (sim->maps_ty != 8 || rest < 1 || rest > kStripTX) return false;
+  return nx < kTX || (sim->coef_form != CF_F32 &&
+                      div_up(nx, kTX) * div_up(ny, 8) > slots_of(sim) / 2);
+}
+
+// CTAs per chunk of a pass.
+long long tiles_of(const Sim *sim, long long nx, long long ny, int ty, bool strip) {
+  if (strip) return nx / kTX * div_up(ny, ty) + div_up(ny, kStripTY);
+  return std::max(1ll, div_up(nx, kTX)) * std::max(1ll, div_up(ny, ty));
 }
 
 }  // namespace
@@ -55,8 +94,8 @@ constexpr long long kLongChunk = 32, kMinChunk = 4;
 FastShape fast_shape(const Sim *sim, long long nx, long long ny, long long nz) {
   const int ty = sim->maps_ty ? sim->maps_ty : chosen_ty(sim->coef_form);
   if (nz < 1) return FastShape{kTX, ty, 1};
-  const long long tiles = std::max(1ll, (nx + kTX - 1) / kTX) * std::max(1ll, (ny + ty - 1) / ty);
-  const long long slots = sim->fast_slots > 0 ? sim->fast_slots : 2 * 152;
+  const long long tiles = tiles_of(sim, nx, ny, ty, !sim->d_energy && has_strip(sim, nx, ny));
+  const long long slots = slots_of(sim);
   const long long one_each = slots / 2;  // two CTAs fit an SM
   long long best_zc = nz, best_cost = -1;
   for (long long c = 1; c <= nz; ++c) {
@@ -81,15 +120,16 @@ FastShape fast_shape(const Sim *sim, long long nx, long long ny, long long nz) {
 int fast_default_ty(int form) { return chosen_ty(form); }
 
 bool fast_encode_pair_maps(const float2 *buf, long long sx, long long sy, long long sz,
-                           long long pitch, int ty, CUtensorMap *halo, CUtensorMap *own,
+                           long long pitch, int tx, int ty, CUtensorMap *halo, CUtensorMap *own,
                            std::string *err) {
+  const uint32_t w = static_cast<uint32_t>(tx);
   const uint64_t dims3[3] = {static_cast<uint64_t>(sx), static_cast<uint64_t>(sy),
                              static_cast<uint64_t>(sz)};
   // (p, q) pair buffers: 8-byte elements
   const uint64_t str8[2] = {static_cast<uint64_t>(pitch) * 8,
                             static_cast<uint64_t>(pitch * sy) * 8};
-  const uint32_t box_halo[3] = {kTX + 8, static_cast<uint32_t>(ty) + 8, kGroup};
-  const uint32_t box_tile[3] = {kTX, static_cast<uint32_t>(ty), kGroup};
+  const uint32_t box_halo[3] = {w + 8, static_cast<uint32_t>(ty) + 8, kGroup};
+  const uint32_t box_tile[3] = {w, static_cast<uint32_t>(ty), kGroup};
   const auto U64 = CU_TENSOR_MAP_DATA_TYPE_UINT64;
   return encode_tiled(halo, buf, 3, dims3, str8, box_halo, err, U64) &&
          encode_tiled(own, buf, 3, dims3, str8, box_tile, err, U64);
@@ -97,19 +137,20 @@ bool fast_encode_pair_maps(const float2 *buf, long long sx, long long sy, long l
 
 bool fast_encode_medium_maps(int form, const float *coef, const void *coef16, const float *vv,
                              const float4 *vbase, long long sx, long long sy, long long sz,
-                             long long pitch, long long count, int ty, CUtensorMap out[4],
-                             std::string *err) {
+                             long long pitch, long long count, int tx, int ty,
+                             CUtensorMap out[4], std::string *err) {
+  const uint32_t w = static_cast<uint32_t>(tx);
   const uint64_t X = sx, Y = sy, Z = sz, P = pitch, PL = pitch * sy;
   const uint64_t dims3[3] = {X, Y, Z};
   const uint64_t str8[2] = {P * 8, PL * 8};
   const uint64_t str4[2] = {P * 4, PL * 4};
-  const uint32_t box_tile[3] = {kTX, static_cast<uint32_t>(ty), kGroup};
+  const uint32_t box_tile[3] = {w, static_cast<uint32_t>(ty), kGroup};
   // 16-byte coefficient groups: two 8-byte elements per point, so a tile
   // row is one 512-byte box row (a box whose innermost extent is a single
   // 16-byte group makes the copy engine walk 32 x TY rows of 16 bytes)
   const uint64_t dims16[3] = {2 * X, Y, Z};
   const uint64_t str16[2] = {P * 16, PL * 16};
-  const uint32_t box16[3] = {2 * kTX, static_cast<uint32_t>(ty), kGroup};
+  const uint32_t box16[3] = {2 * w, static_cast<uint32_t>(ty), kGroup};
   const auto U64 = CU_TENSOR_MAP_DATA_TYPE_UINT64, U32 = CU_TENSOR_MAP_DATA_TYPE_UINT32;
   const long long cnt = count;
   // out[0] = L (cxx, cyy, cxy, czz), out[1] = O1, out[2] = O2, out[3] = the
@@ -151,18 +192,21 @@ bool fast_encode_maps(Sim *sim, std::string *err) {
   // (done here, before any stream capture)
   const int kTY = chosen_ty(sim->coef_form);
   cudaError_t ae = ops_for(sim->coef_form, kTY).attrs();
+  if (ae == cudaSuccess) ae = strip_ops(sim->coef_form).attrs();
   if (ae != cudaSuccess) {
     *err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ae);
     return false;
   }
-  for (int b = 0; b < 2; ++b)
-    if (!fast_encode_pair_maps(sim->pq[b], sim->sx, sim->sy, sim->sz, sim->pitch, kTY,
-                               &sim->tm_halo[b], &sim->tm_own[b], err))
-      return false;
-  if (!fast_encode_medium_maps(sim->coef_form, sim->coef, sim->coef16, sim->vv, sim->vbase,
-                               sim->sx, sim->sy, sim->sz, sim->pitch, sim->count, kTY, sim->tm_c,
-                               err))
-    return false;
+  auto encode = [&](FastMaps &m, int tx, int ty) {
+    for (int b = 0; b < 2; ++b)
+      if (!fast_encode_pair_maps(sim->pq[b], sim->sx, sim->sy, sim->sz, sim->pitch, tx, ty,
+                                 &m.halo[b], &m.own[b], err))
+        return false;
+    return fast_encode_medium_maps(sim->coef_form, sim->coef, sim->coef16, sim->vv, sim->vbase,
+                                   sim->sx, sim->sy, sim->sz, sim->pitch, sim->count, tx, ty, m.c,
+                                   err);
+  };
+  if (!encode(sim->maps, kTX, kTY) || !encode(sim->strip_maps, kStripTX, kStripTY)) return false;
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sim->device) != cudaSuccess)
     sms = 0;
@@ -187,8 +231,27 @@ cudaError_t launch_batch(cudaStream_t st, const BatchLaunch &bl, int ty, int for
   return ops_for(form, ty).launch_batch(st, bl, iso, sponge, blocks);
 }
 
+int fast_launches(const Sim *sim, long long nx, long long ny) {
+  return has_strip(sim, nx, ny) && nx >= kTX ? 2 : 1;
+}
+
 cudaError_t launch_fast(Sim *sim, const StepParams &prm, int cur_buf, int prev_buf) {
-  return ops_for(sim->coef_form, sim->maps_ty).launch(sim, prm, cur_buf, prev_buf);
+  const FastOps &ops = ops_for(sim->coef_form, sim->maps_ty);
+  const long long nx = prm.x1 - prm.tile_x0, ny = prm.y1 - prm.tile_y0;
+  if (!has_strip(sim, nx, ny)) return ops.launch(sim, sim->maps, prm, cur_buf, prev_buf);
+  // the strip first: its few CTAs start with the first wave of the others,
+  // which share no point with it
+  const int cut = prm.tile_x0 + static_cast<int>(nx / kTX * kTX);
+  StepParams p = prm;
+  p.tile_x0 = cut;
+  p.x0 = std::max(prm.x0, cut);
+  const cudaError_t e =
+      strip_ops(sim->coef_form).launch(sim, sim->strip_maps, p, cur_buf, prev_buf);
+  if (e != cudaSuccess || cut == prm.tile_x0) return e;
+  p = prm;
+  p.x1 = cut;
+  p.beside = 1;
+  return ops.launch(sim, sim->maps, p, cur_buf, prev_buf);
 }
 
 }  // namespace dcg

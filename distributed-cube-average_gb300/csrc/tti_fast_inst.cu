@@ -1,6 +1,6 @@
 // tti_fast_inst.cu -- the fast sm_103a Fletcher TTI time step: the kernels of
-// one coefficient form (DC_FORM) and tile height (DC_TY).  The build compiles
-// this file once per pair, in parallel; tti_fast.cu picks the pair.
+// one coefficient form (DC_FORM) and tile shape (DC_TX x DC_TY).  The build
+// compiles this file once per combination, in parallel; tti_fast.cu picks one.
 //
 // One pass updates p and q (the coupled pseudo-acoustic TTI system of the
 // reference, include/sample_compute.h:105-185) for every point of a box.
@@ -125,8 +125,8 @@ struct FastLayout {
   static_assert(H_PLANE % 128 == 0 && L_PLANE % 128 == 0 && O1_PLANE % 128 == 0 &&
                     O2_PLANE % 128 == 0 && VB_PLANE % 128 == 0 && DY_BYTES % 128 == 0,
                 "every TMA destination is 128-byte aligned");
-  static_assert(TX == 32, "half a warp spans one tile row");
-  static_assert(TY % 2 == 0, "a warp owns two tile rows");
+  static constexpr int ROWS = 64 / TX;  // tile rows of a warp (two points per lane)
+  static_assert((TX == 32 || TX == 16) && TY % ROWS == 0, "a warp owns whole tile rows");
 };
 
 // Packed FP32 pair arithmetic (one instruction updates p and q).
@@ -435,8 +435,9 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + Lay::OFF_BAR);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // a warp owns two tile rows, a lane the points tx and tx + 1 of one
-  const int tx = 2 * (lane & 15), ty = 2 * warp + (lane >> 4);
+  // a warp owns ROWS tile rows, a lane the points tx and tx + 1 of one
+  constexpr int ROWS = Lay::ROWS;
+  const int tx = 2 * (lane % (TX / 2)), ty = ROWS * warp + lane / (TX / 2);
   const int n_it = ze - zb + 2 * kHalo;
   const int gx = x0 + tx, gy = y0 + ty;
   const bool row_in = gy >= prm.y0 && gy < prm.y1;
@@ -534,16 +535,19 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
   StageAddr sa;
   sa.halo = sbase + Lay::OFF_H + 8 * ((ty + kHalo) * HX + tx + kHalo);
   // the halo column whose y-derivative this lane computes (four columns on
-  // either side of the warp's two rows; lanes 16-31: of the next plane)
-  const int hrow = 2 * warp + ((lane >> 3) & 1), hcol = (lane & 7) < 4 ? (lane & 7) : TX + (lane & 7);
-  sa.col = sbase + Lay::OFF_H + 8 * ((hrow + kHalo) * HX + hcol) + (lane < 16 ? 0 : Lay::H_PLANE);
+  // either side of the warp's rows; with two rows lanes 16-31 do the next
+  // plane's)
+  const int hrow = ROWS * warp + (lane >> 3) % ROWS;
+  const int hcol = (lane & 7) < 4 ? (lane & 7) : TX + (lane & 7);
+  const bool hnext = ROWS == 2 && lane >= 16;
+  sa.col = sbase + Lay::OFF_H + 8 * ((hrow + kHalo) * HX + hcol) + (hnext ? Lay::H_PLANE : 0);
   sa.t8 = sbase + 8 * (ty * TX + tx);
   sa.t4 = sbase + 4 * (ty * TX + tx);
   sa.t16 = (sbase + 16 * (ty * TX + tx)) ^ ((tid & 4) ? 16u : 0u);
   sa.row = sbase + 16 * ty;
   const uint32_t dy = sbase + Lay::OFF_DY + 8 * (ty * HX + tx + kHalo);
   const uint32_t dycol =
-      sbase + Lay::OFF_DY + 8 * (hrow * HX + hcol) + (lane < 16 ? 0 : Lay::DY_BYTES);
+      sbase + Lay::OFF_DY + 8 * (hrow * HX + hcol) + (hnext ? Lay::DY_BYTES : 0);
   // global position of the first point at the first output plane (advanced
   // by one plane per output; never dereferenced for inactive points)
   float2 *out = prm.prev + (static_cast<long long>(zb) * prm.plane +
@@ -611,9 +615,9 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
                                     w[7 + c], w[c], w[8 + c]);
       }
       sts4<DY>(dy, dyq[8 + u][0], dyq[8 + u][1]);
-      // y-derivatives of the 4 + 4 halo columns (needed by d2/dxdy): of this
-      // plane and the next one at once where the group holds both
-      if (u % 2 == 0 && (u + 1 < GROUP || lane < 16))
+      // y-derivatives of the 4 + 4 halo columns (needed by d2/dxdy): with two
+      // rows of this plane and the next one at once where the group holds both
+      if (ROWS > 2 || (u % 2 == 0 && (u + 1 < GROUP || lane < 16)))
         sts2<DY>(dycol, d1s<ISO, CHAIN>(w1y, lds2<H - 8 * HX>(sa.col), lds2<H + 8 * HX>(sa.col),
                                         lds2<H - 16 * HX>(sa.col), lds2<H + 16 * HX>(sa.col),
                                         lds2<H - 24 * HX>(sa.col), lds2<H + 24 * HX>(sa.col),
@@ -856,27 +860,28 @@ __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
   }
 }
 
-constexpr int kTX = kFastTX, kTY = DC_TY, kCF = DC_FORM;
+constexpr int kTX = DC_TX, kTY = DC_TY, kCF = DC_FORM;
 using Lay = FastLayout<kTX, kTY, kCF>;
 
 template <bool SPONGE, bool ISO>
-cudaError_t launch_fast_t(Sim *sim, const StepParams &prm, int cur_buf, int prev_buf) {
+cudaError_t launch_fast_t(const Sim *sim, const FastMaps &maps, const StepParams &prm,
+                          int cur_buf, int prev_buf) {
   const int nx = prm.x1 - prm.tile_x0, ny = prm.y1 - prm.tile_y0;
   const int nz = prm.z1 - prm.z0;
   dim3 grid((nx + kTX - 1) / kTX, (ny + kTY - 1) / kTY, (nz + prm.zchunk - 1) / prm.zchunk);
-  // tm_c: L, O1, O2, row bases
   return launch_dependent(fast_kernel<kTX, kTY, kCF, SPONGE, ISO>, grid, Lay::NT, Lay::SMEM_BYTES,
-                          sim->stream, sim->tm_halo[cur_buf], sim->tm_own[prev_buf],
-                          sim->tm_c[0], sim->tm_c[1], sim->tm_c[2], sim->tm_c[3], prm);
+                          sim->stream, maps.halo[cur_buf], maps.own[prev_buf], maps.c[0],
+                          maps.c[1], maps.c[2], maps.c[3], prm);
 }
 
-cudaError_t launch_one(Sim *sim, const StepParams &prm, int cur, int prev) {
+cudaError_t launch_one(const Sim *sim, const FastMaps &maps, const StepParams &prm, int cur,
+                       int prev) {
   const bool iso = sim->dx == sim->dy && sim->dy == sim->dz;
   if (prm.sponge)
-    return iso ? launch_fast_t<true, true>(sim, prm, cur, prev)
-               : launch_fast_t<true, false>(sim, prm, cur, prev);
-  return iso ? launch_fast_t<false, true>(sim, prm, cur, prev)
-             : launch_fast_t<false, false>(sim, prm, cur, prev);
+    return iso ? launch_fast_t<true, true>(sim, maps, prm, cur, prev)
+               : launch_fast_t<true, false>(sim, maps, prm, cur, prev);
+  return iso ? launch_fast_t<false, true>(sim, maps, prm, cur, prev)
+             : launch_fast_t<false, false>(sim, maps, prm, cur, prev);
 }
 
 template <typename K>
@@ -906,6 +911,7 @@ int occupancy(K kernel) {
 // instance; the others differ by a few registers, well inside the limit).
 int occ_one() { return occupancy(fast_kernel<kTX, kTY, kCF, true, true>); }
 
+#if DC_TX == 32
 // Batch kernel variants: every coefficient form and spacing with the
 // sponge; without it (all shots' profiles are 1, e.g. learned layers) for
 // equal spacing and the FP32 / FP16 / BF16 forms.
@@ -937,12 +943,18 @@ cudaError_t launch_batch_one(cudaStream_t st, const BatchLaunch &bl, bool iso, b
              : go(batch_kernel<kTX, kTY, kCF, true, false>);
 }
 
+#endif
+
 }  // namespace
 
 template <>
-const FastOps &fast_ops<DC_FORM, DC_TY>() {
+const FastOps &fast_ops<DC_FORM, DC_TX, DC_TY>() {
+#if DC_TX == 32
   static const FastOps ops = {attrs_one, occ_one, launch_one,
                               attrs_batch, occ_batch, launch_batch_one};
+#else
+  static const FastOps ops = {attrs_one, occ_one, launch_one, nullptr, nullptr, nullptr};
+#endif
   return ops;
 }
 

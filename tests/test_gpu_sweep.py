@@ -98,6 +98,40 @@ def test_short_chunks_change_no_bit(dc, monkeypatch, sizes):
         assert np.array_equal(tr, outs[0][1])
 
 
+@pytest.mark.parametrize("medium", ["PRECOMP_F16", "PRECOMP_BF16", "VPZ_VSV"])
+@pytest.mark.parametrize("sizes", [(169, 216, 17), (184, 209, 12), (20, 40, 15), (9, 24, 70)])
+def test_narrow_last_column(dc, monkeypatch, sizes, medium):
+    """Left-over columns in 16 x 16 tiles (1, 16, 12 and 1 of them): the bits of
+    the 32 x 16 tiles, which have no such launch; receivers and the source on
+    both sides of the cut."""
+    form = getattr(dc, "MEDIUM_" + medium)
+    coef, fields = inputs(sizes, 6)
+    sx, sy, sz = sizes
+    cut = 4 + (sx - 8) // 32 * 32
+    xs = sorted({max(4, cut - 2), max(4, cut - 1), min(cut, sx - 5), min(cut + 1, sx - 5), sx - 5})
+    rec = np.array([x + y * sx + z * sx * sy for z in (4, sz // 2, sz - 5) for y in (4, sy - 5)
+                    for x in xs])
+    outs = []
+    for ty in ("8", "16"):
+        monkeypatch.setenv("DC_GB300_FAST_TY", ty)
+        with dc.Simulation(sizes, (12.5,) * 3, 1e-3, medium=form, device=0) as sim:
+            if medium == "VPZ_VSV":
+                sim.set_vpz_vsv(np.sqrt(coef[6]), 0.4 * np.sqrt(coef[7]))
+            else:
+                sim.set_precomp(coef)
+            sim.set_fields(*fields)
+            sim.set_source(int(rec[len(xs) + 2]), np.linspace(1.0, 2.0, 6))
+            sim.set_sponge(*(np.linspace(0.9, 1.0, n) for n in sizes))
+            sim.set_receivers(rec, 5)
+            sim.run(3)
+            sim.propagate_box((4, 5, 4), (sx - 4, sy - 4, sz - 4))
+            sim.run(2)
+            sim.synchronize()
+            outs.append((sim.get_fields(), sim.traces(5)))
+    assert all(np.array_equal(outs[0][0][k], outs[1][0][k]) for k in outs[0][0])
+    assert np.array_equal(outs[0][1], outs[1][1])
+
+
 @pytest.mark.parametrize("medium", ["PRECOMP", "PRECOMP_F16", "VPZ_VSV"])
 def test_boxes_beside_one_another(dc, medium):
     """Disjoint boxes of a step run beside one another, anything else waits:
