@@ -422,7 +422,11 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
                                              const int ze, unsigned char *smem) {
   using Lay = FastLayout<TX, TY, CF>;
   using CB = CoefBytes<CF>;
-  constexpr int GROUP = kGroup;
+  // Planes of the unrolled body: one group, or two in the vpz/vsv form, whose
+  // planes are the shortest (its 408^3 step: 525 -> 516 us; half the queue
+  // moves).  In the other forms two no longer fit the instruction cache
+  // (FP16, 872 x 424 x 268: 30.1 -> 30.8 ms for 24 steps).
+  constexpr int GROUP = kGroup, BODY = CF == CF_VV ? 2 * kGroup : kGroup;
   constexpr int HX = Lay::HX;
   constexpr int NT = Lay::NT;
   constexpr unsigned kAll = 0xffffffffu;
@@ -496,10 +500,10 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
   // Register queues of both columns.  cq, dxq, dyq: centre value, x- and
   // y-derivative of the last eight planes (oldest first) and of the body's
   // own; aq, bq, zq: in-plane part of H1, in-plane Laplacian and czz of the
-  // last four and the body's own.  Moved down by GROUP after every body.
-  float2 cq[8 + GROUP][2], dxq[8 + GROUP][2], dyq[8 + GROUP][2];
-  float2 aq[kHalo + GROUP][2], bq[kHalo + GROUP][2];
-  float zq[kHalo + GROUP][2];
+  // last four and the body's own.  Moved down by BODY after every body.
+  float2 cq[8 + BODY][2], dxq[8 + BODY][2], dyq[8 + BODY][2];
+  float2 aq[kHalo + BODY][2], bq[kHalo + BODY][2];
+  float zq[kHalo + BODY][2];
   float2 e_acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
   bool bad = false;  // a wait of this thread timed out
 
@@ -556,22 +560,23 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
   int sel = 1;        // stage of the current group
   uint32_t par = 1u;  // its mbarrier parity
   sa.shift(Lay::STAGE_BYTES);
-  int it0 = 0;      // first iteration of the body (one group)
+  int it0 = 0;      // first iteration of the body
   int stop = n_it;  // a group boundary where a time-out was seen
 
   // Iteration it0 + u; false past the end of the sweep.
   auto plane = [&](auto U) __attribute__((always_inline)) {
     constexpr int u = decltype(U)::value;
-    constexpr int DY = u * Lay::DY_BYTES;
+    constexpr int g = u % GROUP;  // the plane inside its group
+    constexpr int DY = g * Lay::DY_BYTES;
     if (it0 + u >= n_it) return false;  // CTA-uniform
-    if (u == 0) {
+    if (g == 0) {
       // Every warp has read the previous group: refill its stage with the
       // next one, then wait for the current one.
       if (__syncthreads_or(bad)) {
-        stop = it0;
+        stop = it0 + u;
         return false;
       }
-      if (tid == 0 && it0 + GROUP < n_it) issue(it0 + GROUP, sel);
+      if (tid == 0 && it0 + u + GROUP < n_it) issue(it0 + u + GROUP, sel);
       sa.shift(sel ? -Lay::STAGE_BYTES : Lay::STAGE_BYTES);
       sel ^= 1;
       par ^= sel ^ 1;
@@ -587,7 +592,7 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
     float2 xx[2], yy[2];
     {
       float2 w[10], v[8][2];  // row of the two points; their columns
-      constexpr int H = Lay::OFF_H + u * Lay::H_PLANE;
+      constexpr int H = Lay::OFF_H + g * Lay::H_PLANE;
       ld_pairs<H - 32>(sa.halo, w[0], w[1]);
       ld_pairs<H - 16>(sa.halo, w[2], w[3]);
       ld_pairs<H>(sa.halo, w[4], w[5]);
@@ -617,7 +622,7 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
       sts4<DY>(dy, dyq[8 + u][0], dyq[8 + u][1]);
       // y-derivatives of the 4 + 4 halo columns (needed by d2/dxdy): with two
       // rows of this plane and the next one at once where the group holds both
-      if (ROWS > 2 || (u % 2 == 0 && (u + 1 < GROUP || lane < 16)))
+      if (ROWS > 2 || (g % 2 == 0 && (g + 1 < GROUP || lane < 16)))
         sts2<DY>(dycol, d1s<ISO, CHAIN>(w1y, lds2<H - 8 * HX>(sa.col), lds2<H + 8 * HX>(sa.col),
                                         lds2<H - 16 * HX>(sa.col), lds2<H + 16 * HX>(sa.col),
                                         lds2<H - 24 * HX>(sa.col), lds2<H + 24 * HX>(sa.col),
@@ -630,10 +635,10 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
       constexpr int m4 = u, m3 = u + 1, m2 = u + 2, m1 = u + 3, z0 = u + 4, p1 = u + 5,
                     p2 = u + 6, p3 = u + 7, p4 = u + 8;
       OutMedium md[2];
-      load_out<CF, Lay::OFF_O1 + u * Lay::O1_PLANE, Lay::OFF_O2 + u * Lay::O2_PLANE,
-               Lay::OFF_VB + u * Lay::VB_PLANE>(sa, md);
+      load_out<CF, Lay::OFF_O1 + g * Lay::O1_PLANE, Lay::OFF_O2 + g * Lay::O2_PLANE,
+               Lay::OFF_VB + g * Lay::VB_PLANE>(sa, md);
       float2 pv[2], nv[2];
-      ld_pairs<Lay::OFF_OWN + u * Lay::OWN_PLANE>(sa.t8, pv[0], pv[1]);
+      ld_pairs<Lay::OFF_OWN + g * Lay::OWN_PLANE>(sa.t8, pv[0], pv[1]);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const float2 zz = d2s<ISO, CHAIN>(w2z, cq[z0][c], cq[m1][c], cq[p1][c], cq[m2][c],
@@ -719,7 +724,7 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
       e[4] = dyq[8 + u][0];
       e[5] = dyq[8 + u][1];
       float4 lc[2];
-      load_lead<CF, Lay::OFF_L + u * Lay::L_PLANE>(sa, lc);  // cxx, cyy, cxy, czz
+      load_lead<CF, Lay::OFF_L + g * Lay::L_PLANE>(sa, lc);  // cxx, cyy, cxy, czz
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const float2 xy = d1s<ISO, CHAIN>(w1x, e[3 + c], e[5 + c], e[2 + c], e[6 + c], e[1 + c],
@@ -731,23 +736,25 @@ __device__ __forceinline__ bool sweep_column(const CUtensorMap *tm_cur,
     }
     return true;
   };
-  while (plane(Const<0>{}) && plane(Const<1>{}) && plane(Const<2>{})) {
-    it0 += GROUP;
-    ev -= GROUP;
-    if (SPONGE) gzp += GROUP;
+  while (plane(Const<0>{}) && plane(Const<1>{}) && plane(Const<2>{}) &&
+         (BODY == 3 || (plane(Const<BODY == 3 ? 0 : 3>{}) && plane(Const<BODY == 3 ? 0 : 4>{}) &&
+                        plane(Const<BODY == 3 ? 0 : 5>{})))) {
+    it0 += BODY;
+    ev -= BODY;
+    if (SPONGE) gzp += BODY;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        cq[i][c] = cq[i + GROUP][c];
-        dxq[i][c] = dxq[i + GROUP][c];
-        dyq[i][c] = dyq[i + GROUP][c];
+        cq[i][c] = cq[i + BODY][c];
+        dxq[i][c] = dxq[i + BODY][c];
+        dyq[i][c] = dyq[i + BODY][c];
       }
 #pragma unroll
       for (int i = 0; i < kHalo; ++i) {
-        aq[i][c] = aq[i + GROUP][c];
-        bq[i][c] = bq[i + GROUP][c];
-        zq[i][c] = zq[i + GROUP][c];
+        aq[i][c] = aq[i + BODY][c];
+        bq[i][c] = bq[i + BODY][c];
+        zq[i][c] = zq[i + BODY][c];
       }
     }
   }
