@@ -114,20 +114,18 @@ struct StepParams {
 
 // One launch of the batched fast kernel: up to kMaxBatchShots shots, each a
 // box with its own wavefields, source, sponge and receivers, cropped out of
-// one shared medium.  Work items are column tiles (x, y) x z-chunks of every
-// shot, numbered shot by shot; persistent CTAs stride over them.
+// one shared medium.  A work item is a piece of a column tile: {shot, x tile |
+// y tile << 16, first plane, end plane}; persistent CTAs stride over them.
 constexpr int kMaxBatchShots = 64;
 struct BatchLaunch {
   CUtensorMap tm_l, tm_o1, tm_o2;  // shared medium (coefficient groups)
   CUtensorMap tm_vb;                // FP16 medium: velocity bases per row
   const CUtensorMap *maps;          // [shot][4]: halo of buffer 0, 1; own tile of buffer 0, 1
-  const int *order;                 // launch order of the work items (null: shot by shot)
+  const int4 *items;                // in launch order
   int nshots;
   int cur_buf;                      // buffer holding (pc, qc) in every shot
   int n_items;
   int *err;
-  int item_prefix[kMaxBatchShots + 1];
-  int tiles_x[kMaxBatchShots], tiles_y[kMaxBatchShots];
   StepParams shot[kMaxBatchShots];
 };
 

@@ -832,10 +832,8 @@ __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
   if (prm.beside) grid_dep_wait();
 }
 
-// One step of a batch of shots: persistent CTAs stride over the work items
-// (shot by shot: x tile fastest, then y tile, then z-chunk).  The shot of an
-// item is found from the per-shot prefix counts, so every index here is
-// CTA-uniform.
+// One step of a batch of shots: CTAs stride over the work items, whose shot,
+// tile and planes the host's table gives, so every index here is CTA-uniform.
 template <int TX, int TY, int CF, bool SPONGE, bool ISO>
 __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
     batch_kernel(const __grid_constant__ BatchLaunch bl) {
@@ -845,18 +843,10 @@ __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
     return;
   }
   for (int slot = blockIdx.x; slot < bl.n_items; slot += gridDim.x) {
-    const int item = bl.order ? bl.order[slot] : slot;
-    int s = 0;
-    while (s + 1 < bl.nshots && bl.item_prefix[s + 1] <= item) ++s;
+    const int4 item = bl.items[slot];
+    const int s = item.x, zb = item.z, ze = item.w;
     const StepParams &prm = bl.shot[s];
-    int local = item - bl.item_prefix[s];
-    const int ix = local % bl.tiles_x[s];
-    local /= bl.tiles_x[s];
-    const int iy = local % bl.tiles_y[s];
-    const int iz = local / bl.tiles_y[s];
-    const int x0 = prm.tile_x0 + ix * TX, y0 = prm.tile_y0 + iy * TY;
-    const int zb = prm.z0 + iz * prm.zchunk;
-    const int ze = min(zb + prm.zchunk, prm.z1);
+    const int x0 = prm.tile_x0 + (item.y & 0xffff) * TX, y0 = prm.tile_y0 + (item.y >> 16) * TY;
     const CUtensorMap *m = bl.maps + 4 * s;
     // weights, dt2 and energy (none) are the same in every shot: read them
     // from shot 0 at fixed offsets

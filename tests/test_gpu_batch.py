@@ -295,3 +295,45 @@ def test_batch_many_shots_span_launch_groups(dc, medium_coef):
                 for k in ("pc", "qc", "pp", "qp"):
                     assert np.array_equal(got[i][k], want[k]), (with_layer, i, k)
                 assert np.abs(got[i]["pc"]).max() > 0
+
+
+# (all items cut into four pieces; whole columns, halves and quarters in one
+# launch; columns one plane short of two pieces)
+@pytest.mark.parametrize("count,sizes", [(1, (40, 40, 120)), (9, (101, 72, 107)),
+                                         (12, (136, 72, 55))])
+def test_cut_tail_changes_no_bit(dc, port, count, sizes):
+    from dc_gb300 import medium
+    box = (208, 128, 120)
+    coef = port.precomp(medium.layered_fields(medium.layered_spec(12, box), box))
+    mid = tuple(s // 2 for s in sizes)
+    shots = []
+    for i in range(count):
+        origin = (4 * (i * 5 % ((box[0] - sizes[0]) // 4 + 1)), i * 7 % (box[1] - sizes[1] + 1),
+                  i * 3 % (box[2] - sizes[2] + 1))
+        shots.append((origin, (mid[0] + i, mid[1] - i, mid[2] + i % 3)))
+    rec = [(x, mid[1], z) for x in range(5, sizes[0] - 5, 7) for z in (5, mid[2], sizes[2] - 6)]
+    with dc.Batch(box, D, DT, medium=dc.MEDIUM_PRECOMP, device=0, max_steps=STEPS) as b:
+        b.set_precomp(coef)
+        for i, (origin, src) in enumerate(shots):
+            b.add_shot(sizes, origin, src, 45.0, ABSORB, KAPPA)
+            b.set_receivers(i, rec)
+        b.set_grid(False)
+        b.run(STEPS)
+        b.synchronize()
+        got = [(b.get_fields(i), b.traces(i, STEPS)) for i in range(count)]
+    for (origin, src), (fields, traces) in zip(shots, got):
+        with dc.Simulation(sizes, D, DT, kernel=dc.KERNEL_FAST, medium=dc.MEDIUM_PRECOMP,
+                           device=0) as sim:
+            sim.set_precomp([crop(c, origin, sizes) for c in coef])
+            sim.set_fields()
+            sim.set_source(dense_index(sizes, src), wavelet(dc, 45.0, STEPS + 3))
+            sim.set_sponge(*sponge(dc, sizes))
+            sim.set_receivers([dense_index(sizes, r) for r in rec], STEPS)
+            sim.run(STEPS)
+            sim.synchronize()
+            want = sim.get_fields()
+            assert np.array_equal(traces, sim.traces(STEPS))
+        for k in ("pp", "pc", "qp", "qc"):
+            assert np.array_equal(fields[k], want[k]), k
+        # the wave has reached every plane
+        assert np.abs(fields["pc"][4:-4]).max(axis=(1, 2)).min() > 0
