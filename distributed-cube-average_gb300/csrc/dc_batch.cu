@@ -308,6 +308,7 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
   b->groups.clear();
   b->group_first.clear();
   b->group_branch.clear();
+  long long all_items = 0;  // before cutting
   // launch groups of up to kMaxBatchShots shots, never spanning two chains
   std::vector<std::pair<int, int>> spans;  // [first, last) shots
   for (int br = 0; br < b->nbranch; ++br) {
@@ -378,6 +379,7 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
       if (tx > 0xffff || ty_n > 0x7fff || items > (1ll << 30))
         return fail(DC_GB300_ERR_ARG, "too many work items in a launch");
     }
+    all_items += items;
     b->groups.push_back(bl);
   }
   BATCH_TRY(batch_prepare(ty, b->coef_form));
@@ -402,8 +404,12 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
   // columns otherwise, one CTA per item) the steps were 1.077 times as fast
   // (geometric mean; 1.3 columns per resident CTA: 1.20, 4.0: 1.06, 6.0: 1.01,
   // 13.2: 1.02); a half of the resident CTAs' items in four pieces 1.068, a
-  // half in two 1.058, a quarter in eight alone 0.993.  Two chains fill each other's
-  // ends: with the learned layer cutting cost 0 to 5 %, so not there.
+  // half in two 1.058, a quarter in eight alone 0.993.
+  // Two chains (the learned layer) fill each other's ends: cutting the last
+  // items cost them 0 to 5 % at 1.8 to 5.9 columns per resident CTA.  There
+  // every column is cut alike, so that the step has at least two items per
+  // resident CTA: 0.36 columns each 2.2 times as fast, 0.7 1.5, 1.1 1.15,
+  // 1.6 1.03.
   std::vector<int4> table;
   std::vector<size_t> group_off;
   long long max_items = 0;
@@ -429,10 +435,12 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
       return a.item.x < c.item.x;
     });
     const auto parts = [&](size_t i, int nz) {
-      if (b->nbranch == 2) return 1;
       const size_t left = keys.size() - i, quarter = (resident + 3) / 4;
-      const int n = left <= quarter ? 8 : left <= 3 * quarter ? 2 : 1;
-      return std::min(n, std::max(1, nz / kMinPiece));
+      const long long n = b->nbranch == 2 ? 1 + 2ll * resident / all_items
+                          : left <= quarter     ? 8
+                          : left <= 3 * quarter ? 2
+                                                : 1;
+      return static_cast<int>(std::min<long long>(n, std::max(1, nz / kMinPiece)));
     };
     for (size_t i = 0; i < keys.size(); ++i) {
       const int4 it = keys[i].item;

@@ -337,3 +337,33 @@ def test_cut_tail_changes_no_bit(dc, port, count, sizes):
             assert np.array_equal(fields[k], want[k]), k
         # the wave has reached every plane
         assert np.abs(fields["pc"][4:-4]).max(axis=(1, 2)).min() > 0
+
+
+@pytest.mark.parametrize("sizes", [(48, 44, 101), (44, 40, 57)])  # three pieces; two
+def test_cut_columns_of_two_chains_change_no_bit(dc, port, sizes):
+    from dc_gb300 import learned, medium
+    box, layer, mid = (96, 64, 104), 8, tuple(s // 2 for s in sizes)
+    coef = port.precomp(medium.layered_fields(medium.layered_spec(13, box), box))
+    origins = [(0, 3, 1), (24, 11, 0), (48, 20, 3)]
+    with dc.MLP(device=0, params=np.load(learned.WEIGHTS)) as mlp:
+        with dc.Batch(box, D, DT, device=0, max_steps=STEPS) as b:
+            b.set_precomp(coef)
+            for o in origins:
+                b.add_shot(sizes, o, mid, 45.0, 0, 0.0)
+            b.set_learned_layer(mlp, layer)
+            b.set_grid(False)
+            b.run(STEPS)
+            b.synchronize()
+            got = [b.get_fields(i) for i in range(len(origins))]
+        for o, g in zip(origins, got):
+            with dc.Simulation(sizes, D, DT, kernel=dc.KERNEL_FAST, device=0) as sim:
+                sim.set_precomp([crop(c, o, sizes) for c in coef])
+                sim.set_fields()
+                sim.set_source(dense_index(sizes, mid), wavelet(dc, 45.0, STEPS + 3))
+                dc.set_learned_layer(sim, mlp, layer)
+                sim.run(STEPS)
+                sim.synchronize()
+                want = sim.get_fields()
+            for k in ("pp", "pc", "qp", "qc"):
+                assert np.array_equal(g[k], want[k]), k
+            assert np.abs(g["pc"][4:-4]).max(axis=(1, 2)).min() > 0
