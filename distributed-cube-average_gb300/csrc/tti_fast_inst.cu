@@ -832,9 +832,13 @@ __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
   if (prm.beside) grid_dep_wait();
 }
 
-// One step of a batch of shots: CTAs stride over the work items, whose shot,
-// tile and planes the host's table gives, so every index here is CTA-uniform.
-template <int TX, int TY, int CF, bool SPONGE, bool ISO>
+// One step of a batch of shots: one CTA per work item, or (LOOP) CTAs that
+// stride over them.  The host's table gives an item's shot, tile and planes,
+// so every index here is CTA-uniform.  Two kernels, because around the sweep a
+// loop costs the compiled sweep 12 % more instructions (moves of the queues,
+// addresses worked out again in every plane): eight FP16 shots, 97 M points,
+// 0.964 ms per step with the loop, 0.925 without.
+template <int TX, int TY, int CF, bool SPONGE, bool ISO, bool LOOP>
 __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
     batch_kernel(const __grid_constant__ BatchLaunch bl) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -842,7 +846,9 @@ __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
     if (threadIdx.x == 0) atomicOr(bl.err, kErrAlign);
     return;
   }
-  for (int slot = blockIdx.x; slot < bl.n_items; slot += gridDim.x) {
+  int slot = blockIdx.x;
+  if (slot >= bl.n_items) return;
+  do {
     const int4 item = bl.items[slot];
     const int s = item.x, zb = item.z, ze = item.w;
     const StepParams &prm = bl.shot[s];
@@ -854,7 +860,8 @@ __global__ void __launch_bounds__(TX *TY / 2, kMinBlocks<TX * TY / 2>)
                                                &bl.tm_l, &bl.tm_o1, &bl.tm_o2, &bl.tm_vb, prm,
                                                bl.shot[0], x0, y0, zb, ze, smem))
       return;
-  }
+    slot += gridDim.x;
+  } while (LOOP && slot < bl.n_items);
 }
 
 constexpr int kTX = DC_TX, kTY = DC_TY, kCF = DC_FORM;
@@ -914,30 +921,43 @@ int occ_one() { return occupancy(fast_kernel<kTX, kTY, kCF, true, true>); }
 // equal spacing and the FP32 / FP16 / BF16 forms.
 constexpr bool kNoSponge = kCF != CF_VV;
 
-cudaError_t attrs_batch() {
-  cudaError_t e = allow_smem(batch_kernel<kTX, kTY, kCF, true, false>);
-  if (e == cudaSuccess) e = allow_smem(batch_kernel<kTX, kTY, kCF, true, true>);
+template <bool LOOP>
+cudaError_t attrs_loop() {
+  cudaError_t e = allow_smem(batch_kernel<kTX, kTY, kCF, true, false, LOOP>);
+  if (e == cudaSuccess) e = allow_smem(batch_kernel<kTX, kTY, kCF, true, true, LOOP>);
   if constexpr (kNoSponge)
-    if (e == cudaSuccess) e = allow_smem(batch_kernel<kTX, kTY, kCF, false, true>);
+    if (e == cudaSuccess) e = allow_smem(batch_kernel<kTX, kTY, kCF, false, true, LOOP>);
   return e;
+}
+
+cudaError_t attrs_batch() {
+  const cudaError_t e = attrs_loop<false>();
+  return e == cudaSuccess ? attrs_loop<true>() : e;
 }
 
 int occ_batch(bool iso, bool sponge) {
   if constexpr (kNoSponge)
-    if (iso && !sponge) return occupancy(batch_kernel<kTX, kTY, kCF, false, true>);
-  return iso ? occupancy(batch_kernel<kTX, kTY, kCF, true, true>)
-             : occupancy(batch_kernel<kTX, kTY, kCF, true, false>);
+    if (iso && !sponge) return occupancy(batch_kernel<kTX, kTY, kCF, false, true, true>);
+  return iso ? occupancy(batch_kernel<kTX, kTY, kCF, true, true, true>)
+             : occupancy(batch_kernel<kTX, kTY, kCF, true, false, true>);
 }
 
-cudaError_t launch_batch_one(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
-                             int blocks) {
+template <bool LOOP>
+cudaError_t launch_loop(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
+                        int blocks) {
   auto go = [&](auto kernel) {
     return launch_dependent(kernel, dim3(blocks), Lay::NT, Lay::SMEM_BYTES, st, bl);
   };
   if constexpr (kNoSponge)
-    if (iso && !sponge) return go(batch_kernel<kTX, kTY, kCF, false, true>);
-  return iso ? go(batch_kernel<kTX, kTY, kCF, true, true>)
-             : go(batch_kernel<kTX, kTY, kCF, true, false>);
+    if (iso && !sponge) return go(batch_kernel<kTX, kTY, kCF, false, true, LOOP>);
+  return iso ? go(batch_kernel<kTX, kTY, kCF, true, true, LOOP>)
+             : go(batch_kernel<kTX, kTY, kCF, true, false, LOOP>);
+}
+
+cudaError_t launch_batch_one(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
+                             int blocks) {
+  return blocks < bl.n_items ? launch_loop<true>(st, bl, iso, sponge, blocks)
+                             : launch_loop<false>(st, bl, iso, sponge, bl.n_items);
 }
 
 #endif
