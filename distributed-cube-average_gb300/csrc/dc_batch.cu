@@ -222,7 +222,8 @@ int refresh_narrow(Batch *b) {
   return DC_GB300_OK;
 }
 
-constexpr int kMinPiece = 24;  // planes (each piece streams eight more)
+// Planes of a cut column's piece, one chain and two (each streams eight more).
+constexpr int kMinPiece[2] = {24, 12};
 
 // Builds the device tables and the launch parameters for tile rows `ty`
 // and `zsplit` z-chunks per column.
@@ -398,7 +399,7 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
   //
   // A launch's last items are cut along z: those of the last quarter of the
   // resident CTAs into up to eight pieces, those of the half before into two,
-  // each of at least kMinPiece planes.  Whole columns end a launch with SMs
+  // each of at least 24 planes.  Whole columns end a launch with SMs
   // that have nothing left to do for up to a column's time, and a step is a
   // handful of columns per SM.  Over ten batches of 1 to 15 shots (whole
   // columns otherwise, one CTA per item) the steps were 1.077 times as fast
@@ -409,7 +410,10 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
   // items cost them 0 to 5 % at 1.8 to 5.9 columns per resident CTA.  There
   // every column is cut alike, so that the step has at least two items per
   // resident CTA: 0.36 columns each 2.2 times as fast, 0.7 1.5, 1.1 1.15,
-  // 1.6 1.03.
+  // 1.6 1.03; pieces of down to 12 planes, which over 24 gave 1.08 (nine
+  // batches of 0.2 to 1.2 columns each, 1.0 to 1.25; 16: 1.07, 8: 1.08 with
+  // less at 0.36).  Columns that are split already are brought to about two
+  // items per resident CTA, not past them (three small FP32 batches 3 to 10 %).
   std::vector<int4> table;
   std::vector<size_t> group_off;
   long long max_items = 0;
@@ -434,13 +438,16 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
       if (a.x != c.x) return a.x < c.x;
       return a.item.x < c.item.x;
     });
+    const long long even = zsplit > 1 ? (2ll * resident + all_items / 2) / all_items
+                                      : 1 + 2ll * resident / all_items;
     const auto parts = [&](size_t i, int nz) {
       const size_t left = keys.size() - i, quarter = (resident + 3) / 4;
-      const long long n = b->nbranch == 2 ? 1 + 2ll * resident / all_items
+      const bool two = b->nbranch == 2;
+      const long long n = two                   ? even
                           : left <= quarter     ? 8
                           : left <= 3 * quarter ? 2
                                                 : 1;
-      return static_cast<int>(std::min<long long>(n, std::max(1, nz / kMinPiece)));
+      return static_cast<int>(std::max(1ll, std::min<long long>(n, nz / kMinPiece[two])));
     };
     for (size_t i = 0; i < keys.size(); ++i) {
       const int4 it = keys[i].item;
@@ -455,8 +462,10 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
   BATCH_TRY(cudaMemcpyAsync(b->d_items, table.data(), sizeof(int4) * table.size(),
                             cudaMemcpyHostToDevice, b->stream));
   for (size_t g = 0; g < b->groups.size(); ++g) b->groups[g].items = b->d_items + group_off[g];
-  // persistent CTAs, or one CTA per work item
-  b->blocks = static_cast<int>(b->persistent ? std::min<long long>(max_items, resident) : max_items);
+  // Persistent CTAs, or one CTA per work item.  Up to two items per resident
+  // CTA there is nothing for a loop to save, and the kernel without one is the
+  // faster (a learned step of two small FP16 shots 0.145 ms instead of 0.158).
+  b->blocks = static_cast<int>(b->persistent && max_items > 2ll * resident ? resident : max_items);
   BATCH_TRY(cudaStreamSynchronize(b->stream));
   b->prepared = true;
   return DC_GB300_OK;
