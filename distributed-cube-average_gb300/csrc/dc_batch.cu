@@ -4,7 +4,7 @@
 // absorbing layer and halo) and any number of shots.  Each shot is a box
 // cropped out of the medium at (ox, oy, oz) with its own (p, q) wavefields,
 // source wavelet, sponge and receivers.  One step of all shots is one launch
-// of the persistent batch kernel per group of up to kMaxBatchShots shots;
+// of the batch kernel per group of up to kMaxBatchShots shots;
 // steps are captured into CUDA graphs of kGraphSteps steps.  Tile rows (TY)
 // and the z-split of each column are chosen by dc_gb300_batch_autotune,
 // which times every candidate on the batch itself.

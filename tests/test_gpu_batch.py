@@ -339,7 +339,7 @@ def test_cut_tail_changes_no_bit(dc, port, count, sizes):
         assert np.abs(fields["pc"][4:-4]).max(axis=(1, 2)).min() > 0
 
 
-@pytest.mark.parametrize("sizes", [(48, 44, 101), (44, 40, 57)])  # eight pieces; four
+@pytest.mark.parametrize("sizes", [(48, 44, 101), (44, 40, 57)])  # seven pieces; four
 def test_cut_columns_of_two_chains_change_no_bit(dc, port, sizes):
     from dc_gb300 import learned, medium
     box, layer, mid = (96, 64, 104), 8, tuple(s // 2 for s in sizes)
