@@ -367,3 +367,65 @@ def test_cut_columns_of_two_chains_change_no_bit(dc, port, sizes):
             for k in ("pp", "pc", "qp", "qc"):
                 assert np.array_equal(g[k], want[k]), k
             assert np.abs(g["pc"][4:-4]).max(axis=(1, 2)).min() > 0
+
+
+# (a form, a sponge width and a spacing per compiled kind of sweep)
+@pytest.mark.parametrize("form,absorb,d", [("PRECOMP", ABSORB, D),
+                                           ("PRECOMP", ABSORB, (12.5, 10.0, 8.0)),
+                                           ("PRECOMP_F16", ABSORB, D), ("PRECOMP_F16", 0, D),
+                                           ("PRECOMP_BF16", ABSORB, D)])
+def test_ctas_that_take_several_items(dc, port, form, absorb, d):
+    """699 uneven columns in a launch, more than twice what the GPU holds at
+    once: persistent CTAs take two or three each.  One CTA per item, and
+    single-shot simulations, give the same bits."""
+    from dc_gb300 import medium
+    box, steps = (208, 128, 64), 40
+    coef = port.precomp(medium.layered_fields(medium.layered_spec(17, box), box))
+    kinds = [(136, 72, 40), (101, 80, 33), (73, 61, 47)]
+    shots = []
+    for i in range(26):
+        sizes = kinds[i % 3]
+        origin = (4 * (i * 5 % ((box[0] - sizes[0]) // 4 + 1)), i * 7 % (box[1] - sizes[1] + 1),
+                  i * 3 % (box[2] - sizes[2] + 1))
+        mid = tuple(s // 2 for s in sizes)
+        rec = [(x, mid[1], z) for x in range(5, sizes[0] - 5, 7) for z in (5, mid[2], sizes[2] - 6)]
+        shots.append((sizes, origin, (mid[0] + i % 4, mid[1], mid[2] - i % 3), rec))
+    tiles = sum(-(-(s[0] - 8) // 32) * -(-(s[1] - 8) // 8) for s, _, _, _ in shots)
+    assert tiles == 699
+    outs = {}
+    for grid in (None, True, False):
+        with dc.Batch(box, d, DT, medium=getattr(dc, "MEDIUM_" + form), device=0,
+                      max_steps=steps) as b:
+            b.set_precomp(coef)
+            for i, (sizes, origin, src, rec) in enumerate(shots):
+                b.add_shot(sizes, origin, src, 45.0, absorb, KAPPA if absorb else 0.0)
+                b.set_receivers(i, rec)
+            b.set_tiles(8, 1)
+            if grid is not None:
+                b.set_grid(grid)
+            b.run(steps)
+            b.synchronize()
+            assert b.persistent == (grid is not False)
+            outs[grid] = [(b.get_fields(i), b.traces(i, steps)) for i in range(len(shots))]
+    for grid in (None, True):
+        for (f, tr), (g, tg) in zip(outs[grid], outs[False]):
+            assert all(np.array_equal(f[k], g[k]) for k in ("pp", "pc", "qp", "qc"))
+            assert np.array_equal(tr, tg)
+            assert np.abs(f["pc"][4:-4]).max(axis=(1, 2)).min() > 0
+    if form != "PRECOMP":
+        return  # (the 16-bit encodings are of the whole medium)
+    for i in (0, 12, 25):
+        sizes, origin, src, rec = shots[i]
+        with dc.Simulation(sizes, d, DT, kernel=dc.KERNEL_FAST,
+                           medium=getattr(dc, "MEDIUM_" + form), device=0) as sim:
+            sim.set_precomp([crop(c, origin, sizes) for c in coef])
+            sim.set_fields()
+            sim.set_source(dense_index(sizes, src), wavelet(dc, 45.0, steps + 3))
+            sim.set_sponge(*sponge(dc, sizes))
+            sim.set_receivers([dense_index(sizes, r) for r in rec], steps)
+            sim.run(steps)
+            sim.synchronize()
+            want, want_tr = sim.get_fields(), sim.traces(steps)
+        f, tr = outs[True][i]
+        assert all(np.array_equal(f[k], want[k]) for k in ("pp", "pc", "qp", "qc"))
+        assert np.array_equal(tr, want_tr)
