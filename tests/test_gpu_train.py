@@ -67,3 +67,67 @@ def test_first_adam_step(dc, batch):
     assert np.array_equal(new[g == 0], p[g == 0])
     assert abs(hist[0] - le / lw) <= 1e-5 * le / lw
     assert again[-1] < 0.5 * hist[0]  # and it goes on downhill
+
+
+FULL_GRID = 152 * 16 * 128  # samples of a launch with one pass in every CTA
+
+
+def many_samples(n, seed):
+    """Samples of about the same size, so that each one shows in the sums."""
+    rng = np.random.default_rng(seed)
+    s = np.empty((n, 33), np.float32)
+    s[:, :32] = rng.normal(0, 1, (n, 32)) * rng.uniform(0.5, 2.0, (n, 1))
+    s[:, 32] = rng.integers(0, 8, n)
+    s[1::4, :32] = 0.0
+    return s, rng.normal(0, 1, (n, 2)).astype(np.float32)
+
+
+def parts(m, xs, ts, n):
+    """Gradient and sums of samples [0, n), at most one pass per CTA at a time."""
+    g, le, lw = 0.0, 0.0, 0.0
+    for k in range(0, n, FULL_GRID):
+        gk, (e, w) = m.gradient(xs.data_ptr() + k * 33 * 4, ts.data_ptr() + k * 2 * 4,
+                                min(FULL_GRID, n - k))
+        g, le, lw = g + gk.astype(np.float64), le + e, lw + w
+    return g, le, lw
+
+
+@pytest.mark.parametrize("n", [FULL_GRID + 1, FULL_GRID + 129, 3 * FULL_GRID - 57])
+def test_gradient_of_several_passes_per_cta(dc, n):
+    """Against the same samples in launches of one pass: the same activations;
+    each FP32 sum of 2432 CTAs' partials rounds by some sqrt(2432) 2^-24 = 3e-6
+    of itself, and one sample of 3e5 weighs 1e-3 of a gradient that grows like
+    sqrt(n), 3e-6 of the FP64 sums."""
+    s, t = many_samples(n, n)
+    xs, ts = dev(s), dev(t)
+    with dc.MLP(device=0, params=mo.init_params(3)) as m:
+        g, (le, lw) = m.gradient(xs.data_ptr(), ts.data_ptr(), n)
+        gw, le_w, lw_w = parts(m, xs, ts, n)
+    assert rel_l2(g, gw) <= 2e-5
+    assert abs(lw - lw_w) <= 1e-9 * lw_w and abs(le - le_w) <= 1e-9 * le_w
+
+
+def test_training_step_of_several_passes_per_cta(dc):
+    """A batch past one pass per CTA: its mean loss and the direction of its
+    first Adam step are those of the samples it draws."""
+    n, batch, lr, seed = 4001, FULL_GRID + 129, 2e-3, 11
+    s, t = many_samples(n, 21)
+    mask = (1 << 64) - 1
+    z = np.uint64((seed + 0x9E3779B97F4A7C15) & mask) ^ (
+        np.arange(batch, dtype=np.uint64) * np.uint64(0x2545F4914F6CDD1D))
+    z = z + np.uint64(0x9E3779B97F4A7C15)
+    z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+    z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+    drawn = ((z ^ (z >> np.uint64(31))) % np.uint64(n)).astype(np.int64)
+    p = mo.init_params(5)
+    xs, ts, xd, td = dev(s), dev(t), dev(s[drawn]), dev(t[drawn])
+    with dc.MLP(device=0, params=p) as m:
+        g, le, lw = parts(m, xd, td, batch)
+        hist = m.train(xs.data_ptr(), ts.data_ptr(), n, 1, batch, lr, seed=seed)
+        new = m.params()
+    assert abs(hist[0] - le / lw) <= 2.0 ** -23 * le / lw  # (stored in FP32)
+    g = g / lw
+    big = np.abs(g) > 1e-4
+    assert big.sum() > 500
+    want = p - lr * g / (np.abs(g) + 1e-8)
+    assert np.max(np.abs(new - want)[big]) <= 1e-3 * lr
