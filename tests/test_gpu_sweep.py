@@ -203,3 +203,30 @@ def test_exact_kernel_edges_and_alignment(dc, medium):
         a, b = outs
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
         assert np.allclose(a[2], b[2], rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("even", [True, False])
+@pytest.mark.parametrize("sizes", [(40, 24, 46), (73, 41, 29), (104, 56, 75)])
+def test_fp32_tile_rows_change_no_bit(dc, monkeypatch, sizes, even):
+    """32 x 8 and 32 x 16 tiles of the FP32 form: two CTAs or one per SM, and
+    other columns at the edges."""
+    d = (12.5, 12.5, 12.5) if even else (12.5, 10.0, 8.0)
+    coef, fields = inputs(sizes, 8)
+    sx, sy, sz = sizes
+    rec = np.array([sx // 2 + y * sx + z * sx * sy for z in (4, sz // 2, sz - 5)
+                    for y in (4, sy // 2, sy - 5)])
+    outs = []
+    for ty in ("8", "16"):
+        monkeypatch.setenv("DC_GB300_FAST_TY", ty)
+        with dc.Simulation(sizes, d, 1e-3, medium=dc.MEDIUM_PRECOMP, device=0) as sim:
+            sim.set_precomp(coef)
+            sim.set_fields(*fields)
+            sim.set_source(int(rec[4]), np.linspace(1.0, 2.0, 6))
+            sim.set_sponge(*(np.linspace(0.9, 1.0, n) for n in sizes))
+            sim.set_receivers(rec, 5)
+            sim.run(5)
+            sim.synchronize()
+            outs.append((sim.get_fields(), sim.traces(5)))
+    assert all(np.array_equal(outs[0][0][k], outs[1][0][k]) for k in outs[0][0])
+    assert np.array_equal(outs[0][1], outs[1][1])
+    assert np.abs(outs[0][0]["pc"]).max() > 0
