@@ -84,7 +84,7 @@ T *direct_view(T *p, int dev) {
 // The simulation of an API call.  Any call but a propagate ends the run of
 // boxes that may be computed beside one another.
 Sim *impl(dc_gb300_sim *h) {
-  if (h && h->impl) h->impl->boxes.clear();
+  if (h && h->impl) h->impl->n_boxes = 0;
   return h ? h->impl : nullptr;
 }
 
@@ -1394,15 +1394,17 @@ namespace {
 // share no point with it, so none reads what another writes.  Notes the box.
 bool runs_beside(Sim *s, const long long b0[3], const long long b1[3]) {
   const dc_device_data &a = s->handle->abi;
-  if (a.pp != s->box_pp || a.pc != s->box_pc) s->boxes.clear();
+  if (a.pp != s->box_pp || a.pc != s->box_pc || s->n_boxes == Sim::kMaxBeside) s->n_boxes = 0;
   s->box_pp = a.pp;
   s->box_pc = a.pc;
-  bool apart = !s->boxes.empty() && !s->stream_shared;
-  for (const auto &o : s->boxes)
-    apart = apart && (b0[0] >= o[3] || o[0] >= b1[0] || b0[1] >= o[4] || o[1] >= b1[1] ||
-                      b0[2] >= o[5] || o[2] >= b1[2]);
-  if (!apart) s->boxes.clear();  // this pass waits for all before it
-  s->boxes.push_back({b0[0], b0[1], b0[2], b1[0], b1[1], b1[2]});
+  bool apart = s->n_boxes > 0 && !s->stream_shared;
+  for (int i = 0; i < s->n_boxes && apart; ++i) {
+    const auto &o = s->boxes[i];
+    apart = b0[0] >= o[3] || o[0] >= b1[0] || b0[1] >= o[4] || o[1] >= b1[1] || b0[2] >= o[5] ||
+            o[2] >= b1[2];
+  }
+  if (!apart) s->n_boxes = 0;  // this pass waits for all before it
+  s->boxes[s->n_boxes++] = {b0[0], b0[1], b0[2], b1[0], b1[1], b1[2]};
   return apart;
 }
 
@@ -1423,7 +1425,7 @@ int propagate_box(Sim *s, const size_t start[3], const size_t end[3]) {
   StepParams p;
   if (s->kernel == DC_GB300_KERNEL_FAST) {
     // (a 16-bit copy of the medium is refreshed first)
-    if (s->coef16 && s->coef16_stale) s->boxes.clear();
+    if (s->coef16 && s->coef16_stale) s->n_boxes = 0;
     const int rc = refresh_narrow(s);
     if (rc != DC_GB300_OK) return rc;
     p = make_params(s, b0, b1, s->dx, s->dy, s->dz, s->dt);

@@ -230,3 +230,32 @@ def test_fp32_tile_rows_change_no_bit(dc, monkeypatch, sizes, even):
     assert all(np.array_equal(outs[0][0][k], outs[1][0][k]) for k in outs[0][0])
     assert np.array_equal(outs[0][1], outs[1][1])
     assert np.abs(outs[0][0]["pc"]).max() > 0
+
+
+def test_many_boxes_in_a_step(dc):
+    """A step in boxes of one point: the bits of one box, and the last calls
+    take the host no longer than the first."""
+    import time
+
+    sizes = (40, 40, 32)
+    sx, sy, sz = sizes
+    coef, fields = inputs(sizes, 10)
+    out, took = [], []
+    for split in (False, True):
+        with dc.Simulation(sizes, (12.5,) * 3, 1e-3, device=0) as sim:
+            sim.set_precomp(coef)
+            sim.set_fields(*fields)
+            if not split:
+                sim.propagate_box((4, 4, 4), tuple(s - 4 for s in sizes))
+            else:
+                for z in range(4, sz - 4):
+                    for y in range(4, sy - 4):
+                        t = time.perf_counter()
+                        for x in range(4, sx - 4):
+                            sim.propagate_box((x, y, z), (x + 1, y + 1, z + 1))
+                        took.append(time.perf_counter() - t)
+            sim.synchronize()
+            out.append(sim.get_fields())
+    assert all(np.array_equal(out[0][k], out[1][k]) for k in out[0])
+    # (rows of 32 calls; the first hundred may still fill the launch queue)
+    assert np.median(took[-100:]) <= 2.0 * np.median(took[50:150])
