@@ -1802,6 +1802,15 @@ extern "C" int dc_gb300_exact_steps_noalloc(const dc_gb300_config *cfg, float *p
   if (cfg->medium != DC_GB300_MEDIUM_PRECOMP && cfg->medium != DC_GB300_MEDIUM_VPZ_VSV)
     return dcg::fail(DC_GB300_ERR_ARG,
                 "dc_gb300_exact_steps_noalloc takes the precomp or vpz/vsv medium form");
+  // the kernels read (p, q) and (vpz, vsv) pairs as 8-byte values and the
+  // grouped coefficients as 16-byte ones
+  const size_t medium_align = cfg->medium == DC_GB300_MEDIUM_PRECOMP ? 16 : 8;
+  if (reinterpret_cast<uintptr_t>(pairs[0]) % 8 != 0 ||
+      reinterpret_cast<uintptr_t>(pairs[1]) % 8 != 0 ||
+      reinterpret_cast<uintptr_t>(medium) % medium_align != 0)
+    return dcg::fail(DC_GB300_ERR_ARG,
+                "dc_gb300_exact_steps_noalloc: pairs must be 8-byte aligned, the medium 16-byte "
+                "(precomp) or 8-byte (vpz/vsv) aligned");
   if (!(cfg->dx > 0 && cfg->dy > 0 && cfg->dz > 0 && cfg->dt > 0))
     return dcg::fail(DC_GB300_ERR_ARG, "dx, dy, dz and dt must be positive");
   int ndev = 0;

@@ -497,8 +497,8 @@ template <int MEDIUM, bool SPONGE>
 cudaError_t launch_exact_t(Sim *sim, const StepParams &prm) {
   const int ny = prm.y1 - prm.y0, nz = prm.z1 - prm.z0;
   const int chunks = (nz + prm.zchunk - 1) / prm.zchunk;
-  // pitch and plane are multiples of four pairs; a caller's own buffers may
-  // start anywhere a float may
+  // pitch and plane are multiples of four pairs; a caller's own buffers need
+  // only be aligned to one pair
   const auto base = reinterpret_cast<uintptr_t>(prm.cur);
   if (base % 16 == 0) {
     const int nx = prm.x1 - (prm.x0 & ~1);

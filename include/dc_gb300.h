@@ -532,10 +532,13 @@ int dc_gb300_lb_rollout(dc_gb300_sim *wide, dc_gb300_sim *thin, const long offse
  *           DC_GB300_MEDIUM_VPZ_VSV
  *   pairs   {previous, current}: two device buffers of interleaved (p, q)
  *           pairs, pitch = round_up(sx, 4) points per row, sy*sz rows --
- *           the layout of dc_device_data; on return pairs[1] holds the
+ *           the layout of dc_device_data, 8-byte aligned (faster where the
+ *           current one is 16-byte aligned); on return pairs[1] holds the
  *           newest field and pairs[0] the one before it
- *   medium  device buffer in the grouped coefficient layout (PRECOMP) or
- *           of (vpz, vsv) pairs (VPZ_VSV), same pitch
+ *   medium  device buffer in the grouped coefficient layout (PRECOMP,
+ *           16-byte aligned) or of (vpz, vsv) pairs (VPZ_VSV, 8-byte
+ *           aligned), same pitch; other alignments fail with
+ *           DC_GB300_ERR_ARG
  *   steps   0 .. 4096 (the scratch maximum); larger counts fail with
  *           DC_GB300_ERR_ARG and an explanatory message
  *   energy  host array of `steps` doubles receiving the per-step energy

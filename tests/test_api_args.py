@@ -74,3 +74,18 @@ def test_noalloc_rejects_before_touching_the_device(dc, lib):
     assert lib.dc_gb300_exact_steps_noalloc(C.byref(fast), pairs, C.c_void_p(48), 1, None,
                                             None) == dc.ERR_ARG
     assert lib.dc_gb300_exact_steps_noalloc(None, pairs, None, 1, None, None) == dc.ERR_ARG
+
+
+@pytest.mark.parametrize("form,first,second,medium", [
+    ("PRECOMP", 4, 32, 48), ("PRECOMP", 16, 36, 48), ("PRECOMP", 2, 32, 48),
+    ("PRECOMP", 16, 32, 56), ("PRECOMP", 8, 24, 52), ("VPZ_VSV", 8, 24, 52),
+    ("VPZ_VSV", 12, 24, 56)])
+def test_noalloc_rejects_misaligned_buffers(dc, lib, form, first, second, medium):
+    """The kernels read (p, q) and (vpz, vsv) pairs as 8-byte values and the
+    grouped coefficients as 16-byte ones."""
+    cfg = dc.Config(20, 20, 20, 12.5, 12.5, 12.5, 1e-3, dc.KERNEL_EXACT,
+                    getattr(dc, "MEDIUM_" + form), 0)
+    pairs = (C.c_void_p * 2)(first, second)
+    assert lib.dc_gb300_exact_steps_noalloc(C.byref(cfg), pairs, C.c_void_p(medium), 1, None,
+                                            None) == dc.ERR_ARG
+    assert "aligned" in _err(lib)
