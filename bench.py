@@ -30,7 +30,7 @@ absorbing layers and halos: an 872 x 872 x 616 medium box), each shot a
 crop of U(192, 320) x U(192, 320) x 256 interior cells around its source
 (sources on an 8 x 8 surface grid with seeded jitter, depth 20, Ricker peak
 U(15, 25) Hz), a 48-cell sponge per shot, FP16 medium storage, 64 receivers
-per shot; tile rows, z-split and grid (persistent CTAs or one CTA per tile)
+per shot; tile rows, z-split and grid (persistent CTAs or one CTA per item)
 chosen by the library's autotuner.  One step advances every shot (one
 launch); K defaults to 1000 steps.
 ``value`` is shot-point-updates per second summed over the shots.
@@ -716,8 +716,8 @@ def batch_shots(n_shots: int, seed: int = BATCH_SEED, model=BATCH_MODEL, pad: in
 
 
 def run_batched(args, rank, world, local):
-    """The batched form: all shots in one persistent, graph-captured launch
-    per step.  Ranks > 0 run their own independent batch (weak scaling)."""
+    """The batched form: all shots in one graph-captured launch per step.
+    Ranks > 0 run their own independent batch (weak scaling)."""
     import torch
     import __graft_entry__ as ge
     dc = ge.package()
@@ -744,10 +744,10 @@ def run_batched(args, rank, world, local):
         (ty, zsplit), tune_ms = b.tiles(), None
     else:
         ty, zsplit, tune_ms = b.autotune(3)
-    persistent = b.persistent
     pts = b.points
     b.run(args.warmup)
     b.synchronize()
+    persistent = b.persistent
     stream = torch.cuda.ExternalStream(b.stream)
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     l0 = b.launches
@@ -1002,10 +1002,10 @@ def run_best(args, rank, world, local):
         b.add_shot(sh["sizes"], sh["origin"], sh["src"], sh["fcut"], 0, 0.0)
         b.set_receivers(k, sh["rec"])
     ty, zsplit, _ = b.autotune(3)
-    persistent = b.persistent
     b.set_learned_layer(mlp, layer)
     b.run(args.warmup)
     b.synchronize()
+    persistent = b.persistent
     l0 = b.launches
     with ClockSampler(local) as clk:
         ms = timed_run(b, args.steps)

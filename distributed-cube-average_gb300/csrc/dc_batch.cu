@@ -31,6 +31,10 @@ namespace {
 
 constexpr int kGraphSteps = 32;  // steps per captured graph (even)
 
+// Grid of the stencil launches: one CTA per work item, persistent CTAs, or
+// (until the caller chooses) the faster of the two by the number of items.
+constexpr int kGridItems = 0, kGridPersistent = 1, kGridByRule = 2;
+
 struct BShot {
   dc_gb300_shot cfg;
   long long pitch = 0, plane = 0, count = 0;
@@ -66,10 +70,11 @@ struct Batch {
   std::vector<long long> trace_off;  // per shot, in floats
   int *d_step = nullptr, *d_err = nullptr;
   std::vector<BatchLaunch> groups;   // one launch per group of shots
-  int blocks = 0;
   bool prepared = false;
   int ty = 8, zsplit = 1;
-  bool persistent = true;  // persistent CTAs, or one CTA per work item
+  int grid = kGridByRule;  // the choice of grid, and with the tables made:
+  bool loop = true;        // persistent CTAs (else one CTA per work item),
+  int blocks = 0;          // this many at most
   bool sponge = true;      // some shot's sponge profile differs from 1
   int steps_done = 0;
   int src_applied_step = -1;
@@ -225,9 +230,9 @@ int refresh_narrow(Batch *b) {
 // Planes of a cut column's piece, one chain and two (each streams eight more).
 constexpr int kMinPiece[2] = {24, 12};
 
-// Builds the device tables and the launch parameters for tile rows `ty`
-// and `zsplit` z-chunks per column.
-int prepare(Batch *b, int ty, int zsplit, bool persistent) {
+// Builds the device tables and the launch parameters for tile rows `ty`,
+// `zsplit` z-chunks per column and the choice of grid `grid`.
+int prepare(Batch *b, int ty, int zsplit, int grid) {
   if (!b->medium_set) return fail(DC_GB300_ERR_STATE, "batch medium not set");
   if (b->shots.empty()) return fail(DC_GB300_ERR_STATE, "batch has no shots");
   int rc = refresh_narrow(b);
@@ -235,7 +240,7 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
   free_tables(b);
   b->ty = ty;
   b->zsplit = zsplit;
-  b->persistent = persistent;
+  b->grid = grid;
   const int n = static_cast<int>(b->shots.size());
   std::string err;
   CUtensorMap tm_c[4];
@@ -462,10 +467,12 @@ int prepare(Batch *b, int ty, int zsplit, bool persistent) {
   BATCH_TRY(cudaMemcpyAsync(b->d_items, table.data(), sizeof(int4) * table.size(),
                             cudaMemcpyHostToDevice, b->stream));
   for (size_t g = 0; g < b->groups.size(); ++g) b->groups[g].items = b->d_items + group_off[g];
-  // Persistent CTAs, or one CTA per work item.  Up to two items per resident
-  // CTA there is nothing for a loop to save, and the kernel without one is the
-  // faster (a learned step of two small FP16 shots 0.145 ms instead of 0.158).
-  b->blocks = static_cast<int>(b->persistent && max_items > 2ll * resident ? resident : max_items);
+  // Persistent CTAs, or one CTA per work item, as the caller asks.  By rule up to
+  // two items per resident CTA there is nothing for a loop to save, and the kernel
+  // without one is the faster (a learned step of two small FP16 shots 0.145 ms
+  // instead of 0.158).
+  b->loop = grid == kGridByRule ? max_items > 2ll * resident : grid == kGridPersistent;
+  b->blocks = static_cast<int>(b->loop ? std::min<long long>(resident, max_items) : max_items);
   BATCH_TRY(cudaStreamSynchronize(b->stream));
   b->prepared = true;
   return DC_GB300_OK;
@@ -485,7 +492,10 @@ cudaError_t queue_chain(Batch *b, int cur, int j, int br, cudaStream_t st) {
       bl.shot[k].prev = b->shots[b->group_first[g] + k].pq[1 - cur];  // written in place
     }
     ++b->launches;
-    const cudaError_t e = launch_batch(st, bl, b->ty, b->coef_form, iso, b->sponge, b->blocks);
+    // (a group of few items has one CTA for each, whatever the rule took)
+    const bool loop = b->grid == kGridPersistent || bl.n_items > b->blocks;
+    const cudaError_t e = launch_batch(st, bl, b->ty, b->coef_form, iso, b->sponge, loop,
+                                       std::min(b->blocks, bl.n_items));
     if (e != cudaSuccess) return e;
   }
   if (b->lb_cells > 0) {  // the chain's learned layers, after its stencil launches
@@ -537,7 +547,7 @@ int check_err(Batch *b) {
 // steps, then single launches.
 int run_steps(Batch *b, int steps) {
   if (!b->prepared) {
-    const int rc = prepare(b, b->ty, b->zsplit, b->persistent);
+    const int rc = prepare(b, b->ty, b->zsplit, b->grid);
     if (rc != DC_GB300_OK) return rc;
   }
   if (b->steps_done + steps > b->max_steps)
@@ -920,7 +930,7 @@ extern "C" int dc_gb300_batch_autotune(dc_gb300_batch *h, int steps, int *ty_out
   const int tys[2] = {8, 16};
   const int splits[4] = {1, 2, 4, 8};
   int best_ty = b->ty, best_split = b->zsplit;
-  bool best_persistent = b->persistent;
+  int best_grid = b->grid;
   float best = -1.0f;
   cudaEvent_t e0, e1;
   BATCH_TRY(cudaEventCreate(&e0));
@@ -928,8 +938,10 @@ extern "C" int dc_gb300_batch_autotune(dc_gb300_batch *h, int steps, int *ty_out
   int rc = DC_GB300_OK;
   for (int t : tys) {
     for (int zs : splits) {
-     for (int pers = 1; pers >= 0; --pers) {
-      rc = dcg::prepare(b, t, zs, pers != 0);
+     // by rule, and one CTA per item where the rule takes persistent CTAs
+     for (int grid : {dcg::kGridByRule, dcg::kGridItems}) {
+      if (grid == dcg::kGridItems && !b->loop) continue;
+      rc = dcg::prepare(b, t, zs, grid);
       if (rc != DC_GB300_OK) break;
       rc = dcg::reset_state(b);
       if (rc != DC_GB300_OK) break;
@@ -952,7 +964,7 @@ extern "C" int dc_gb300_batch_autotune(dc_gb300_batch *h, int steps, int *ty_out
         best = ms;
         best_ty = t;
         best_split = zs;
-        best_persistent = pers != 0;
+        best_grid = grid;
       }
      }
      if (rc != DC_GB300_OK) break;
@@ -962,7 +974,7 @@ extern "C" int dc_gb300_batch_autotune(dc_gb300_batch *h, int steps, int *ty_out
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc != DC_GB300_OK) return rc;
-  rc = dcg::prepare(b, best_ty, best_split, best_persistent);
+  rc = dcg::prepare(b, best_ty, best_split, best_grid);
   if (rc != DC_GB300_OK) return rc;
   rc = dcg::reset_state(b);
   if (rc != DC_GB300_OK) return rc;
@@ -1071,14 +1083,18 @@ extern "C" int dc_gb300_batch_set_grid(dc_gb300_batch *h, int persistent) {
   Batch *b = dcg::impl(h);
   if (!b) return fail(DC_GB300_ERR_ARG, "null batch");
   BATCH_TRY(cudaSetDevice(b->device));
-  b->persistent = persistent != 0;
+  b->grid = persistent != 0 ? dcg::kGridPersistent : dcg::kGridItems;
   b->prepared = false;
   dcg::drop_graphs(b);
   return DC_GB300_OK;
 }
 
 extern "C" int dc_gb300_batch_grid(const dc_gb300_batch *h) {
-  return h ? (h->impl.persistent ? 1 : 0) : -1;
+  if (!h) return -1;
+  const Batch &b = h->impl;
+  // (by rule: what the tables were made for, else the default's name)
+  if (b.grid == dcg::kGridByRule) return b.prepared && !b.loop ? 0 : 1;
+  return b.grid;
 }
 
 extern "C" int dc_gb300_batch_tiles(const dc_gb300_batch *h, int *ty, int *zsplit) {

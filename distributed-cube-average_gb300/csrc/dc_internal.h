@@ -115,7 +115,8 @@ struct StepParams {
 // One launch of the batched fast kernel: up to kMaxBatchShots shots, each a
 // box with its own wavefields, source, sponge and receivers, cropped out of
 // one shared medium.  A work item is a piece of a column tile: {shot, x tile |
-// y tile << 16, first plane, end plane}; persistent CTAs stride over them.
+// y tile << 16, first plane, end plane}; one CTA takes each, or persistent CTAs
+// stride over them.
 constexpr int kMaxBatchShots = 64;
 struct BatchLaunch {
   CUtensorMap tm_l, tm_o1, tm_o2;  // shared medium (coefficient groups)
@@ -239,7 +240,7 @@ struct FastOps {
   cudaError_t (*batch_attrs)();
   int (*batch_occupancy)(bool iso, bool sponge);
   cudaError_t (*launch_batch)(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
-                              int blocks);
+                              bool loop, int blocks);
 };
 constexpr int kFastTX = 32;                // tile width: half a warp of two-point lanes
 constexpr int kStripTX = 16, kStripTY = 16;  // tiles of a narrow last column
@@ -297,12 +298,13 @@ bool fast_encode_medium_maps(int form, const float *coef, const void *coef16, co
                              const float4 *vbase, long long sx, long long sy, long long sz,
                              long long pitch, long long count, int tx, int ty,
                              CUtensorMap out[4], std::string *err);
-// Batched fast kernel (always with the sponge).  `blocks` = persistent CTAs.
+// Batched fast kernel: `blocks` CTAs, one per work item, or (`loop`) striding over
+// the items.
 cudaError_t batch_prepare(int ty, int form);  // shared-memory attributes
 // `sponge` false: every shot's sponge profile is 1 (the no-sponge sweep)
 int batch_blocks_per_sm(int ty, int form, bool iso, bool sponge);
 cudaError_t launch_batch(cudaStream_t st, const BatchLaunch &bl, int ty, int form, bool iso,
-                         bool sponge, int blocks);
+                         bool sponge, bool loop, int blocks);
 
 // Launchers.  Return the cudaError_t of the launch.
 cudaError_t launch_fast(Sim *sim, const StepParams &prm, int cur_buf,

@@ -227,8 +227,8 @@ int batch_blocks_per_sm(int ty, int form, bool iso, bool sponge) {
 }
 
 cudaError_t launch_batch(cudaStream_t st, const BatchLaunch &bl, int ty, int form, bool iso,
-                         bool sponge, int blocks) {
-  return ops_for(form, ty).launch_batch(st, bl, iso, sponge, blocks);
+                         bool sponge, bool loop, int blocks) {
+  return ops_for(form, ty).launch_batch(st, bl, iso, sponge, loop, blocks);
 }
 
 int fast_launches(const Sim *sim, long long nx, long long ny) {

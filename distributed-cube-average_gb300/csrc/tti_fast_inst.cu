@@ -955,9 +955,9 @@ cudaError_t launch_loop(cudaStream_t st, const BatchLaunch &bl, bool iso, bool s
 }
 
 cudaError_t launch_batch_one(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
-                             int blocks) {
-  return blocks < bl.n_items ? launch_loop<true>(st, bl, iso, sponge, blocks)
-                             : launch_loop<false>(st, bl, iso, sponge, bl.n_items);
+                             bool loop, int blocks) {
+  return loop ? launch_loop<true>(st, bl, iso, sponge, blocks)
+              : launch_loop<false>(st, bl, iso, sponge, blocks);
 }
 
 #endif

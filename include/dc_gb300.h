@@ -372,8 +372,8 @@ void dc_gb300_sponge_profile(long s, long a, double kappa, float *g);
  * cropped out of the medium, with its own (p, q) wavefields, wavelet, sponge
  * and receivers, stepped exactly as a dc_gb300_sim with the fast kernel
  * steps its cube (bit-identical fields for the same cropped medium).  One
- * step of all shots is one launch of a persistent kernel per 64 shots;
- * runs are captured into CUDA graphs. */
+ * step of all shots is one launch per 64 shots (two chains of launches with
+ * a learned layer); runs are captured into CUDA graphs. */
 typedef struct dc_gb300_batch dc_gb300_batch;
 
 typedef struct {
@@ -410,16 +410,21 @@ int dc_gb300_batch_set_receivers(dc_gb300_batch *batch, int shot, int count, con
 struct dc_gb300_mlp;
 int dc_gb300_batch_set_learned_layer(dc_gb300_batch *batch, const struct dc_gb300_mlp *mlp,
                                      int layer);
-/* Tile rows (8 or 16) and z-chunks per column (1..64). */
+/* Tile rows (8 or 16) and z-chunks per column (1..64); a launch's last
+ * columns, and with a learned layer those of a small batch, are cut further. */
 int dc_gb300_batch_set_tiles(dc_gb300_batch *batch, int ty, int zsplit);
 int dc_gb300_batch_tiles(const dc_gb300_batch *batch, int *ty, int *zsplit);
 /* Grid of the batch kernel: persistent CTAs striding over the work items
- * (1, the default) or one CTA per work item (0).  dc_gb300_batch_grid
- * returns the current choice. */
+ * (1) or one CTA per work item (0).  Until it is set, and where
+ * dc_gb300_batch_autotune leaves it so, a batch takes persistent CTAs when a
+ * launch has more than two items per CTA that the GPU holds at once, else one
+ * CTA per item.  dc_gb300_batch_grid returns what was set, else what the
+ * batch's launches have (1 before its first run or autotune, and after a
+ * change of shots, receivers, tiles or layer until the next). */
 int dc_gb300_batch_set_grid(dc_gb300_batch *batch, int persistent);
 int dc_gb300_batch_grid(const dc_gb300_batch *batch);
-/* Times every candidate -- tile rows x z-split x grid (persistent or one
- * CTA per work item) -- for `steps` steps on this batch, keeps the fastest
+/* Times every candidate -- tile rows x z-split x grid (by the rule above, and
+ * one CTA per work item where that differs) -- for `steps` steps on this batch, keeps the fastest
  * (ms per step in *ms; the grid choice via dc_gb300_batch_grid) and returns
  * the batch to step 0 with zero wavefields and traces: call it before the
  * first run. */

@@ -429,3 +429,30 @@ def test_ctas_that_take_several_items(dc, port, form, absorb, d):
         f, tr = outs[True][i]
         assert all(np.array_equal(f[k], want[k]) for k in ("pp", "pc", "qp", "qc"))
         assert np.array_equal(tr, want_tr)
+
+
+def test_grid_is_the_one_that_runs(dc, medium_coef, batch_f32):
+    """A grid that is set is the one reported and run; until then a batch of
+    few items has one CTA for each, and says so, tuned or not."""
+    with dc.Batch(MEDIUM, D, DT, device=0, max_steps=STEPS + 2) as b:
+        b.set_precomp(medium_coef)
+        for i, (sizes, origin, src, fcut) in enumerate(SHOTS):
+            b.add_shot(sizes, origin, src, fcut, ABSORB, KAPPA)
+            b.set_receivers(i, receivers(sizes, src))
+        b.run(2)
+        assert not b.persistent
+        b.set_grid(True)
+        assert b.persistent
+        b.run(2)
+        assert b.persistent
+        b.autotune(1)
+        assert not b.persistent
+        b.set_grid(False)
+        b.run(1)
+        assert not b.persistent
+        b.set_grid(True)
+        b.run(STEPS - 1)
+        b.synchronize()
+        assert b.persistent
+        for i in range(len(SHOTS)):
+            assert np.array_equal(b.get_fields(i)["pc"], batch_f32[i][0]["pc"])
