@@ -671,7 +671,7 @@ extern "C" int dc_gb300_batch_create(const dc_gb300_batch_config *cfg, dc_gb300_
                  : cfg->medium == DC_GB300_MEDIUM_PRECOMP_BF16 ? dcg::CF_BF16
                                                                : dcg::CF_F32;
   b->max_steps = cfg->max_steps;
-  b->ty = dcg::fast_default_ty(b->coef_form);
+  b->ty = dcg::fast_default_ty();
   auto bail = [&](int code, const std::string &msg) {
     dcg::release(b);
     delete h;
@@ -910,7 +910,7 @@ extern "C" int dc_gb300_batch_set_learned_layer(dc_gb300_batch *h, const dc_gb30
 extern "C" int dc_gb300_batch_set_tiles(dc_gb300_batch *h, int ty, int zsplit) {
   Batch *b = dcg::impl(h);
   if (!b) return fail(DC_GB300_ERR_ARG, "null batch");
-  if (!dcg::fast_tile_rows_valid(ty, b->coef_form) || zsplit < 1 || zsplit > 64)
+  if (!dcg::fast_tile_rows_valid(ty) || zsplit < 1 || zsplit > 64)
     return fail(DC_GB300_ERR_ARG,
                 "tile rows must be 8 or 16 and zsplit in [1, 64]");
   BATCH_TRY(cudaSetDevice(b->device));

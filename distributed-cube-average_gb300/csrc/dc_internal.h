@@ -192,7 +192,7 @@ struct Sim {
   // tensor maps for the fast kernel: its tiles, and the strip's
   FastMaps maps, strip_maps;
   int fast_slots = 0;      // fast-sweep CTAs resident on the device at once
-  int maps_tx = 0, maps_ty = 0;
+  int maps_ty = 0;
   // learned absorbing layer, applied after every stencil pass of a run
   const float *lb_params = nullptr;  // MLP compute parameters (device, owned by the MLP)
   int4 *d_lb_cells = nullptr;        // layer-cell table (recorded rollout steps)
@@ -236,7 +236,7 @@ struct FastOps {
   int (*occupancy)();      // CTAs per SM
   cudaError_t (*launch)(const Sim *sim, const FastMaps &maps, const StepParams &prm, int cur_buf,
                         int prev_buf);
-  // (32-column tiles only)
+  // (32-column tiles of the forms that a batch takes: not vpz/vsv)
   cudaError_t (*batch_attrs)();
   int (*batch_occupancy)(bool iso, bool sponge);
   cudaError_t (*launch_batch)(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
@@ -258,19 +258,8 @@ DCG_DECL_OPS(CF_VV);
 DCG_DECL_OPS(CF_F16);
 DCG_DECL_OPS(CF_BF16);
 #undef DCG_DECL_OPS
+
 constexpr int kGroup = 3;    // planes of a TMA copy, and between two CTA barriers
-template <int FORM, int TY>
-const FastOps &fast_ops();
-#define DCG_DECL_OPS(f)              \
-  template <>                        \
-  const FastOps &fast_ops<f, 8>();   \
-  template <>                        \
-  const FastOps &fast_ops<f, 16>()
-DCG_DECL_OPS(CF_F32);
-DCG_DECL_OPS(CF_VV);
-DCG_DECL_OPS(CF_F16);
-DCG_DECL_OPS(CF_BF16);
-#undef DCG_DECL_OPS
 
 // Fast-kernel tile geometry (chosen at compile time; see tti_fast.cu).
 struct FastShape {
@@ -281,11 +270,10 @@ FastShape fast_shape(const Sim *sim, long long nx, long long ny, long long nz);
 bool fast_encode_maps(Sim *sim, std::string *err);
 // Kernel launches of a fast pass over nx columns (from tile_x0) and ny rows.
 int fast_launches(const Sim *sim, long long nx, long long ny);
-// Tile rows (TY) of the fast kernel for coefficient form `form`: 8 unless
-// DC_GB300_FAST_TY selects 16.
-int fast_default_ty(int form);
-// Whether tile rows `ty` are compiled for coefficient form `form` (8 and 16).
-bool fast_tile_rows_valid(int ty, int form);
+// Tile rows (TY) of the fast kernel: 8 unless DC_GB300_FAST_TY selects 16.
+int fast_default_ty();
+// Whether tile rows `ty` are compiled (8 and 16).
+bool fast_tile_rows_valid(int ty);
 // Tensor maps of one (p, q) pair buffer for tiles of tx x ty: the halo box
 // (read as the current field) and the own tile (previous field).
 bool fast_encode_pair_maps(const float2 *buf, long long sx, long long sy, long long sz,

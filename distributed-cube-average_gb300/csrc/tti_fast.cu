@@ -38,7 +38,7 @@ const FastOps &strip_ops(int form) {
 // 256 threads per SM nothing runs while the CTA waits at its barrier or fills
 // its queues (616^3 FP32 step 2.19 vs 2.31 ms, 872 x 872 x 616 FP16 3.79 vs
 // 4.35, 408^3 vpz/vsv 0.54 vs 0.62, 104^3 shot 2.3 vs 3.2 ms).  DC_GB300_FAST_TY=16 selects 32 x 16.
-int chosen_ty(int) {
+int chosen_ty() {
   const char *e = std::getenv("DC_GB300_FAST_TY");
   const int v = e ? std::atoi(e) : 0;
   return v == 16 ? 16 : 8;
@@ -66,7 +66,7 @@ bool has_strip(const Sim *sim, long long nx, long long ny) {
 }
 
 // CTAs per chunk of a pass.
-long long tiles_of(const Sim *sim, long long nx, long long ny, int ty, bool strip) {
+long long tiles_of(long long nx, long long ny, int ty, bool strip) {
   if (strip) return nx / kTX * div_up(ny, ty) + div_up(ny, kStripTY);
   return std::max(1ll, div_up(nx, kTX)) * std::max(1ll, div_up(ny, ty));
 }
@@ -92,9 +92,9 @@ long long tiles_of(const Sim *sim, long long nx, long long ny, int ty, bool stri
 constexpr long long kLongChunk = 32, kMinChunk = 4;
 
 FastShape fast_shape(const Sim *sim, long long nx, long long ny, long long nz) {
-  const int ty = sim->maps_ty ? sim->maps_ty : chosen_ty(sim->coef_form);
+  const int ty = sim->maps_ty ? sim->maps_ty : chosen_ty();
   if (nz < 1) return FastShape{kTX, ty, 1};
-  const long long tiles = tiles_of(sim, nx, ny, ty, !sim->d_energy && has_strip(sim, nx, ny));
+  const long long tiles = tiles_of(nx, ny, ty, !sim->d_energy && has_strip(sim, nx, ny));
   const long long slots = slots_of(sim);
   const long long one_each = slots / 2;  // two CTAs fit an SM
   long long best_zc = nz, best_cost = -1;
@@ -117,7 +117,7 @@ FastShape fast_shape(const Sim *sim, long long nx, long long ny, long long nz) {
   return FastShape{kTX, ty, static_cast<int>(best_zc)};
 }
 
-int fast_default_ty(int form) { return chosen_ty(form); }
+int fast_default_ty() { return chosen_ty(); }
 
 bool fast_encode_pair_maps(const float2 *buf, long long sx, long long sy, long long sz,
                            long long pitch, int tx, int ty, CUtensorMap *halo, CUtensorMap *own,
@@ -190,7 +190,7 @@ bool fast_encode_medium_maps(int form, const float *coef, const void *coef16, co
 bool fast_encode_maps(Sim *sim, std::string *err) {
   // dynamic shared memory above 48 KB must be enabled per kernel and device
   // (done here, before any stream capture)
-  const int kTY = chosen_ty(sim->coef_form);
+  const int kTY = chosen_ty();
   cudaError_t ae = ops_for(sim->coef_form, kTY).attrs();
   if (ae == cudaSuccess) ae = strip_ops(sim->coef_form).attrs();
   if (ae != cudaSuccess) {
@@ -213,12 +213,11 @@ bool fast_encode_maps(Sim *sim, std::string *err) {
   const int per_sm = ops_for(sim->coef_form, kTY).occupancy();
   sim->fast_slots = sms > 0 && per_sm > 0 ? sms * per_sm : 0;
   cudaGetLastError();  // a failed occupancy query leaves the fallback slot count
-  sim->maps_tx = kTX;
   sim->maps_ty = kTY;
   return true;
 }
 
-bool fast_tile_rows_valid(int ty, int) { return ty == 8 || ty == 16; }
+bool fast_tile_rows_valid(int ty) { return ty == 8 || ty == 16; }
 
 cudaError_t batch_prepare(int ty, int form) { return ops_for(form, ty).batch_attrs(); }
 

@@ -229,10 +229,6 @@ constexpr float kCxy = 0.4546487134f, kCyz = 0.8414709848f;
 constexpr float kCxz = 0.5403023059f;
 constexpr float kV2pxFactor = 1.48f, kV2pnFactor = 1.2f;
 
-struct Medium {
-  float cxx, cyy, cxy, czz, cxz, cyz, v2px, v2pz, v2sz, v2pn;
-};
-
 __device__ __forceinline__ float2 h2f(uint32_t v, bool bf16) {
   if (bf16) {  // bfloat16 -> float: the 16 bits are the float's high half
     return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
@@ -915,63 +911,64 @@ int occupancy(K kernel) {
 // instance; the others differ by a few registers, well inside the limit).
 int occ_one() { return occupancy(fast_kernel<kTX, kTY, kCF, true, true>); }
 
-#if DC_TX == 32
-// Batch kernel variants: every coefficient form and spacing with the
-// sponge; without it (all shots' profiles are 1, e.g. learned layers) for
-// equal spacing and the FP32 / FP16 / BF16 forms.
-constexpr bool kNoSponge = kCF != CF_VV;
+// Batch kernel variants: either spacing with the sponge; without it (all shots'
+// profiles are 1, e.g. learned layers) equal spacing.
+template <int CF>
+struct BatchOps {
+  template <bool LOOP>
+  static cudaError_t attrs_loop() {
+    cudaError_t e = allow_smem(batch_kernel<kTX, kTY, CF, true, false, LOOP>);
+    if (e == cudaSuccess) e = allow_smem(batch_kernel<kTX, kTY, CF, true, true, LOOP>);
+    if (e == cudaSuccess) e = allow_smem(batch_kernel<kTX, kTY, CF, false, true, LOOP>);
+    return e;
+  }
 
-template <bool LOOP>
-cudaError_t attrs_loop() {
-  cudaError_t e = allow_smem(batch_kernel<kTX, kTY, kCF, true, false, LOOP>);
-  if (e == cudaSuccess) e = allow_smem(batch_kernel<kTX, kTY, kCF, true, true, LOOP>);
-  if constexpr (kNoSponge)
-    if (e == cudaSuccess) e = allow_smem(batch_kernel<kTX, kTY, kCF, false, true, LOOP>);
-  return e;
+  static cudaError_t attrs() {
+    const cudaError_t e = attrs_loop<false>();
+    return e == cudaSuccess ? attrs_loop<true>() : e;
+  }
+
+  static int occ(bool iso, bool sponge) {
+    if (iso && !sponge) return occupancy(batch_kernel<kTX, kTY, CF, false, true, true>);
+    return iso ? occupancy(batch_kernel<kTX, kTY, CF, true, true, true>)
+               : occupancy(batch_kernel<kTX, kTY, CF, true, false, true>);
+  }
+
+  template <bool LOOP>
+  static cudaError_t launch_loop(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
+                                 int blocks) {
+    auto go = [&](auto kernel) {
+      return launch_dependent(kernel, dim3(blocks), Lay::NT, Lay::SMEM_BYTES, st, bl);
+    };
+    if (iso && !sponge) return go(batch_kernel<kTX, kTY, CF, false, true, LOOP>);
+    return iso ? go(batch_kernel<kTX, kTY, CF, true, true, LOOP>)
+               : go(batch_kernel<kTX, kTY, CF, true, false, LOOP>);
+  }
+
+  static cudaError_t launch(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
+                            bool loop, int blocks) {
+    return loop ? launch_loop<true>(st, bl, iso, sponge, blocks)
+                : launch_loop<false>(st, bl, iso, sponge, blocks);
+  }
+};
+
+template <int TX, int CF>
+FastOps make_ops() {
+  FastOps ops = {attrs_one, occ_one, launch_one, nullptr, nullptr, nullptr};
+  if constexpr (TX == 32 && CF != CF_VV) {  // what a batch runs
+    using B = BatchOps<CF>;
+    ops.batch_attrs = B::attrs;
+    ops.batch_occupancy = B::occ;
+    ops.launch_batch = B::launch;
+  }
+  return ops;
 }
-
-cudaError_t attrs_batch() {
-  const cudaError_t e = attrs_loop<false>();
-  return e == cudaSuccess ? attrs_loop<true>() : e;
-}
-
-int occ_batch(bool iso, bool sponge) {
-  if constexpr (kNoSponge)
-    if (iso && !sponge) return occupancy(batch_kernel<kTX, kTY, kCF, false, true, true>);
-  return iso ? occupancy(batch_kernel<kTX, kTY, kCF, true, true, true>)
-             : occupancy(batch_kernel<kTX, kTY, kCF, true, false, true>);
-}
-
-template <bool LOOP>
-cudaError_t launch_loop(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
-                        int blocks) {
-  auto go = [&](auto kernel) {
-    return launch_dependent(kernel, dim3(blocks), Lay::NT, Lay::SMEM_BYTES, st, bl);
-  };
-  if constexpr (kNoSponge)
-    if (iso && !sponge) return go(batch_kernel<kTX, kTY, kCF, false, true, LOOP>);
-  return iso ? go(batch_kernel<kTX, kTY, kCF, true, true, LOOP>)
-             : go(batch_kernel<kTX, kTY, kCF, true, false, LOOP>);
-}
-
-cudaError_t launch_batch_one(cudaStream_t st, const BatchLaunch &bl, bool iso, bool sponge,
-                             bool loop, int blocks) {
-  return loop ? launch_loop<true>(st, bl, iso, sponge, blocks)
-              : launch_loop<false>(st, bl, iso, sponge, blocks);
-}
-
-#endif
 
 }  // namespace
 
 template <>
 const FastOps &fast_ops<DC_FORM, DC_TX, DC_TY>() {
-#if DC_TX == 32
-  static const FastOps ops = {attrs_one, occ_one, launch_one,
-                              attrs_batch, occ_batch, launch_batch_one};
-#else
-  static const FastOps ops = {attrs_one, occ_one, launch_one, nullptr, nullptr, nullptr};
-#endif
+  static const FastOps ops = make_ops<kTX, kCF>();
   return ops;
 }
 
