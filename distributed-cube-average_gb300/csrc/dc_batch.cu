@@ -227,7 +227,8 @@ int refresh_narrow(Batch *b) {
   return DC_GB300_OK;
 }
 
-// Planes of a cut column's piece, one chain and two (each streams eight more).
+// Least average planes of a cut column's pieces, one chain and two (each piece
+// streams eight more).
 constexpr int kMinPiece[2] = {24, 12};
 
 // Builds the device tables and the launch parameters for tile rows `ty`,
@@ -403,8 +404,9 @@ int prepare(Batch *b, int ty, int zsplit, int grid) {
   // so the order changes no result.
   //
   // A launch's last items are cut along z: those of the last quarter of the
-  // resident CTAs into up to eight pieces, those of the half before into two,
-  // each of at least 24 planes.  Whole columns end a launch with SMs
+  // resident CTAs into up to eight pieces, those of the half before into two, of
+  // 24 planes or more on average (all but the last have the average rounded up:
+  // 97 planes give 25, 25, 25 and 22).  Whole columns end a launch with SMs
   // that have nothing left to do for up to a column's time, and a step is a
   // handful of columns per SM.  Over ten batches of 1 to 15 shots (whole
   // columns otherwise, one CTA per item) the steps were 1.077 times as fast

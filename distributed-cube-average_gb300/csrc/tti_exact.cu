@@ -13,12 +13,13 @@
 //
 // Data path: a lane owns two x-adjacent columns and sweeps a chunk of z; a CTA
 // covers 32 x 8 columns.  The stencil reads go through the read-only data
-// cache as (p, q) pairs, so this kernel is bound by L1 bandwidth and
-// instruction issue, not HBM: per two points the x-y and x-z terms read eight
-// rows of ten pairs in five 16-byte loads each, the y-z term one 16-byte load
-// per position (149 loads; one point per thread took 217 8-byte loads per
-// point), and packed f32x2 operations round p and q as scalar ones do.  It is
-// the parity anchor, not the throughput path.
+// cache as (p, q) pairs, so this kernel is bound by the L1's data pipe and its
+// latency, not HBM (168 x 168 x 152: 75 % of the pipe's wavefronts, 5.6 of 8 stall
+// cycles per instruction on its loads, issue 31 %, DRAM 1.3 TB/s): per two points
+// the x-y and x-z terms read eight rows of ten pairs in five 16-byte loads each,
+// the y-z term one 16-byte load per position (149 loads; one point per thread took
+// 217 8-byte loads per point), and packed f32x2 operations round p and q as scalar
+// ones do.  It is the parity anchor, not the throughput path.
 #include "dc_internal.h"
 
 namespace dcg {
@@ -301,9 +302,9 @@ __device__ __forceinline__ float2 update_point(const StepParams &prm, const Poin
 }
 
 // Tile of a CTA: 16 lanes of two columns x 8 rows.  Three CTAs per SM: the
-// loads' latency is what is left to hide (168^3 box, 8 steps: 1.34 ms; without
-// the bound two CTAs fit, 1.55 ms, four spill a little, 1.38; one point per
-// thread 1.63).
+// loads' latency is what is left to hide (168 x 168 x 152, 8 steps: 1.34 ms; without
+// the bound two CTAs fit, 1.55 ms; four, with 128 registers for 168, 1.38; one point
+// per thread 1.63).  Three spill 0 to 28 bytes a thread, four 4 to 36.
 constexpr int kPairTX = 32, kPairTY = 8;
 
 template <int MEDIUM, bool SPONGE>

@@ -1,6 +1,6 @@
 """Batched shots (dc_gb300_batch_*): boxes cropped out of one shared medium,
 each with its own wavelet, sponge and receivers, advanced together by the
-persistent batch kernel.
+batch kernel.
 
 * Each shot's fields and traces are bit-identical to a single-shot
   simulation (fast kernel) over the same cropped medium, sponge, wavelet and
